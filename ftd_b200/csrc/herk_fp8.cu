@@ -46,24 +46,8 @@ __global__ void __launch_bounds__(256) qc_to_planes_kernel(const uint8_t* __rest
     const int rl = l / chunks;
     const int t0 = (l - rl * chunks) << 4;
     const int64_t r = r0 + rl;
-    const uint8_t* src = qc + r * K + t0;
     uint32_t w[4];
-    if (vec && t0 + 16 <= K) {
-      const uint4 v = __ldg(reinterpret_cast<const uint4*>(src));
-      w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w;
-    } else {
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        uint32_t acc = 0;
-#pragma unroll
-        for (int b = 0; b < 4; ++b) {
-          const int t = t0 + 4 * q + b;
-          const uint32_t byte = (t < K) ? uint32_t(__ldg(src + 4 * q + b)) : 0u;
-          acc |= byte << (8 * b);
-        }
-        w[q] = acc;
-      }
-    }
+    load_qc16(qc + r * K, t0, K, vec, w);
     uint32_t re[4], im[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) qc4_to_e4m3(w[q], re[q], im[q]);
@@ -94,24 +78,8 @@ __global__ void __launch_bounds__(256) qc_to_planes_s8_kernel(const uint8_t* __r
     const int rl = l / chunks;
     const int t0 = (l - rl * chunks) << 4;
     const int64_t r = r0 + rl;
-    const uint8_t* src = qc + r * K + t0;
     uint32_t w[4];
-    if (vec && t0 + 16 <= K) {
-      const uint4 v = __ldg(reinterpret_cast<const uint4*>(src));
-      w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w;
-    } else {
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        uint32_t acc = 0;
-#pragma unroll
-        for (int b = 0; b < 4; ++b) {
-          const int t = t0 + 4 * q + b;
-          const uint32_t byte = (t < K) ? uint32_t(__ldg(src + 4 * q + b)) : 0u;
-          acc |= byte << (8 * b);
-        }
-        w[q] = acc;
-      }
-    }
+    load_qc16(qc + r * K, t0, K, vec, w);
     uint32_t re[4], im[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) qc4_to_s8(w[q], re[q], im[q]);
@@ -143,24 +111,8 @@ __global__ void __launch_bounds__(256) qc_to_planes6_kernel(const uint8_t* __res
     const int g = l - rl * chunks;
     const int t0 = g << 4;
     const int64_t r = r0 + rl;
-    const uint8_t* src = qc + r * K + t0;
     uint32_t w[4];
-    if (vec && t0 + 16 <= K) {
-      const uint4 v = __ldg(reinterpret_cast<const uint4*>(src));
-      w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w;
-    } else {
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        uint32_t acc = 0;
-#pragma unroll
-        for (int b = 0; b < 4; ++b) {
-          const int t = t0 + 4 * q + b;
-          const uint32_t byte = (t < K) ? uint32_t(__ldg(src + 4 * q + b)) : 0u;
-          acc |= byte << (8 * b);
-        }
-        w[q] = acc;
-      }
-    }
+    load_qc16(qc + r * K, t0, K, vec, w);
     uint32_t re[4], im[4], pr[3], pi[3];
 #pragma unroll
     for (int q = 0; q < 4; ++q) qc4_to_e3m2(w[q], re[q], im[q]);
@@ -267,24 +219,8 @@ __global__ void __launch_bounds__(256) gather_qc_to_planes_kernel(const GatherDe
     const int t0 = (l - rl * chunks) << 4;
     const int r = r0 + rl;
     const int64_t src_row = g.active ? int64_t(__ldg(g.active + r)) : int64_t(r);
-    const uint8_t* src = g.a + src_row * g.lda + t0;
     uint32_t w[4];
-    if (vec && t0 + 16 <= g.k) {
-      const uint4 v = __ldg(reinterpret_cast<const uint4*>(src));
-      w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w;
-    } else {
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        uint32_t acc = 0;
-#pragma unroll
-        for (int b = 0; b < 4; ++b) {
-          const int t = t0 + 4 * q + b;
-          const uint32_t byte = (t < g.k) ? uint32_t(__ldg(src + 4 * q + b)) : 0u;
-          acc |= byte << (8 * b);
-        }
-        w[q] = acc;
-      }
-    }
+    load_qc16(g.a + src_row * g.lda, t0, g.k, vec, w);
     uint32_t re[4], im[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) qc4_to_e4m3(w[q], re[q], im[q]);
@@ -1215,14 +1151,24 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kHerkThreads, 1)
 }
 
 // ------------------------------------------------------------------ launchers
-static int rows_per_block(int chunks) {
-  int r = 8192 / (chunks > 0 ? chunks : 1);
-  return r < 1 ? 1 : r;
+// Rows per block of a promotion pass over `rows` rows of `chunks` per-thread
+// pieces: about eight blocks of 256 threads for each of 148 SMs while the
+// problem has that many, at most 32 pieces per thread (rows stay together, and
+// fewer blocks start) and at least one.  One fixed size of 8192 pieces gave
+// 32 channels of 128 x 256 eight blocks (21.9 us of promotion) and 16 of
+// 1024 x 1024 FP16 samples 256 (24.6 us).
+static int rows_per_block(int64_t rows, int chunks) {
+  constexpr int64_t kBlocks = 8 * 148;
+  const int64_t most = 8192 / chunks, least = (256 + chunks - 1) / chunks;
+  int64_t r = rows / kBlocks;
+  if (r < least) r = least;
+  if (r > most) r = most;
+  return r < 1 ? 1 : int(r);
 }
 
 cudaError_t launch_qc_to_planes(const uint8_t* qc, uint8_t* z, int64_t rows, int K, int Kp,
                                 cudaStream_t s, bool neg_plane) {
-  const int rpb = rows_per_block(Kp >> 4);
+  const int rpb = rows_per_block(rows, Kp >> 4);
   const int64_t blocks = (rows + rpb - 1) / rpb;
   qc_to_planes_kernel<<<unsigned(blocks), 256, 0, s>>>(qc, z, rows, K, Kp, rpb, neg_plane ? 1 : 0);
   return cudaGetLastError();
@@ -1230,7 +1176,7 @@ cudaError_t launch_qc_to_planes(const uint8_t* qc, uint8_t* z, int64_t rows, int
 
 cudaError_t launch_qc_to_planes_s8(const uint8_t* qc, uint8_t* z, int64_t rows, int K, int Kp,
                                    cudaStream_t s, bool neg_plane) {
-  const int rpb = rows_per_block(Kp >> 4);
+  const int rpb = rows_per_block(rows, Kp >> 4);
   const int64_t blocks = (rows + rpb - 1) / rpb;
   qc_to_planes_s8_kernel<<<unsigned(blocks), 256, 0, s>>>(qc, z, rows, K, Kp, rpb,
                                                            neg_plane ? 1 : 0);
@@ -1239,7 +1185,7 @@ cudaError_t launch_qc_to_planes_s8(const uint8_t* qc, uint8_t* z, int64_t rows, 
 
 cudaError_t launch_qc_to_planes6(const uint8_t* qc, uint8_t* z, int64_t rows, int K, int Kp,
                                  cudaStream_t s, bool neg_plane) {
-  const int rpb = rows_per_block(Kp >> 4);
+  const int rpb = rows_per_block(rows, Kp >> 4);
   const int64_t blocks = (rows + rpb - 1) / rpb;
   qc_to_planes6_kernel<<<unsigned(blocks), 256, 0, s>>>(qc, z, rows, K, Kp, rpb,
                                                          neg_plane ? 1 : 0);
@@ -1257,7 +1203,7 @@ cudaError_t launch_negate_plane(uint8_t* z, int64_t plane_bytes, int sm_count, c
 
 cudaError_t launch_fp16_to_planes(const void* a16, uint8_t* z, int64_t rows, int K, int Kp,
                                   cudaStream_t s) {
-  const int rpb = rows_per_block(Kp >> 3);
+  const int rpb = rows_per_block(rows, Kp >> 3);
   const int64_t blocks = (rows + rpb - 1) / rpb;
   fp16_to_planes_kernel<<<unsigned(blocks), 256, 0, s>>>(
       static_cast<const __half2*>(a16), z, rows, K, Kp, rpb,
@@ -1267,7 +1213,7 @@ cudaError_t launch_fp16_to_planes(const void* a16, uint8_t* z, int64_t rows, int
 
 cudaError_t launch_gather_qc_to_planes(const GatherDesc* g, int nch, int max_n, uint8_t* z,
                                        int64_t total_rows, int Kp, cudaStream_t s, int neg_plane) {
-  const int rpb = rows_per_block(Kp >> 4);
+  const int rpb = rows_per_block(total_rows, Kp >> 4);
   const dim3 grid(unsigned((max_n + rpb - 1) / rpb), unsigned(nch));
   gather_qc_to_planes_kernel<<<grid, 256, 0, s>>>(g, z, total_rows, Kp, rpb, neg_plane);
   return cudaGetLastError();
