@@ -191,6 +191,72 @@ ftdx_status prepare(ftdx_handle h, const HerkCall& c, cudaStream_t s, const Plan
   return get_plan(h, c.N, int(Kp / kStageK), c.batch, s, plan, pair, splits, c.out_format == 1);
 }
 
+// Strategy of a call on a handle whose user has set none: the single-CTA
+// kernel, with the promotion fused in or not and K split or not, whichever a
+// small model of the device time puts first.  Its terms, in us, fitted to
+// 35 shapes of 1 to 2112 tiles and 2 to 512 k-blocks on 148 SMs (the pick is
+// within 11% of the best split and kernel tried at each, most within 3%):
+//   a tile of b k-blocks takes max(0.75 b, 2.6) + 0.8 -- the MMAs or the
+//     stores, then the pipeline's fill; 1.25 b with the conversion fused in;
+//   the separate promotion 3 for its launch + the planes' bytes at 5.5 TB/s;
+//   split-K 6 for its reduction + the partial triangles at 3 TB/s.
+// 256 inputs x 65536 samples x 4 channels (12 tiles): 408 us unsplit with the
+// promotion apart, 70 us as 12 ranges with it fused in; 128 x 256 x 32: 14.3
+// apart, 10 fused in; 512 x 1024 x 30 (300 tiles): 37.3 apart, 39.3 fused in.
+// The choice depends on sizes and on `fused` alone, so that a call prepared
+// for capture (ftdx_init_herk) finds its plan.
+Strategy auto_strategy(const ftdx_context& h, int N, int K, int batch, bool fused_ok,
+                       bool split_ok) {
+  const int64_t nb = (N + kTile - 1) / kTile, tiles = nb * (nb + 1) / 2 * batch;
+  const int64_t kb = round_up(K, kStageK) / kStageK;
+  const double planes = 3.0 * N * double(batch) * double(kb * kStageK);
+  const double partial = 4.0 * N * (N + 1.0) * batch;  // bytes of one split's triangles
+  Strategy best;
+  // past eight tiles per SM the last round costs little and partials much
+  const int64_t most = split_ok && tiles <= 8 * h.sm_count ? std::min<int64_t>(32, kb) : 1;
+  double best_us = 0;
+  for (int sp = 1; sp <= int(most) && (sp == 1 || sp * partial <= 256e6); ++sp) {
+    const double b = double((kb + sp - 1) / sp);
+    const double rounds = double((tiles * sp + h.sm_count - 1) / h.sm_count);
+    const double sum = sp > 1 ? 6.0 + 0.2 * sp + sp * partial / 3e6 : 0.0;
+    const double apart = 3.0 + planes / 5.5e6 + rounds * (std::max(0.75 * b, 2.6) + 0.8) + sum;
+    const double in_one = rounds * (std::max(1.25 * b, 2.6) + 0.8) + sum;
+    const bool f = fused_ok && in_one < apart;
+    const double us = f ? in_one : apart;
+    if (sp == 1 || us < best_us) {
+      best = Strategy{f ? kStoreFused : 0, 0, sp};
+      best_us = us;
+    }
+  }
+  return best;
+}
+
+Strategy untuned_strategy(ftdx_handle h, const HerkCall& c) {
+  if (h->user_strategy || is_fp4(c)) return h->default_strategy;
+  return auto_strategy(*h, c.N, c.K, c.batch, fused_ok(c), !c.comp && c.out_format == 0);
+}
+
+// Before an untuned call: everything that calls of its shape may need under a
+// later capture, whatever their input's alignment or entry point -- two
+// planes, and the tile plans and partial triangles of the strategies that
+// auto_strategy picks.  Where the partial triangles do not fit, *strat
+// becomes the unsplit kernel.
+ftdx_status prepare_auto(ftdx_handle h, const HerkCall& c, cudaStream_t s, Strategy* strat) {
+  if (h->user_strategy || is_fp4(c) || stream_capturing(s)) return FTDX_OK;
+  const Plan* plan = nullptr;
+  ftdx_status st = prepare(h, c, s, &plan);
+  for (int f = 0; f < 2 && st == FTDX_OK; ++f) {
+    const Strategy a = auto_strategy(*h, c.N, c.K, c.batch, f == 1, true);
+    if (a.splits <= 1) continue;
+    st = prepare(h, c, s, &plan, false, a.splits);
+    if (st == FTDX_ERR_ALLOC) {
+      *strat = Strategy{};
+      return FTDX_OK;
+    }
+  }
+  return st;
+}
+
 // Promotion kernel + correlator kernel on stream s.
 ftdx_status launch_all(ftdx_handle h, const HerkCall& c, const Strategy& strat, cudaStream_t s) {
   if (is_fp4(c)) return launch_fp4(h, c, strat, s);
@@ -370,6 +436,11 @@ ftdx_status run_graph(ftdx_handle h, const HerkCall& c, const Strategy& strat, c
 }
 
 }  // namespace
+
+void clear_strategy(ftdx_handle h) {
+  h->default_strategy = Strategy{};
+  h->user_strategy = false;
+}
 
 std::vector<Strategy> default_candidates(ftdx_handle h, bool fp32_out, bool pair_ok) {
   std::vector<Strategy> v;
@@ -561,18 +632,23 @@ ftdx_status ftdx_herk(ftdx_handle h, const void* A, void* C, int N, int K, int b
   if (e != cudaSuccess) return cuda_fail(h, e, "cudaSetDevice");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const bool capturing = stream_capturing(s);
-  Strategy strat = h->default_strategy;
+  Strategy strat = untuned_strategy(h, c);
+  bool tuned = false;
   if (tune) {
     auto it = h->tuned.find(tune_key(h, c));
     if (it != h->tuned.end()) {
       strat = it->second.st;
+      tuned = true;
     } else if (beta == 0.f && !capturing) {
       TuneEntry te;
       st = run_tune(h, c, s, &te);
       if (st != FTDX_OK) return st;
       strat = te.st;
+      tuned = true;
     }
   }
+  if (!tuned) st = prepare_auto(h, c, s, &strat);
+  if (st != FTDX_OK) return st;
   if (h->graph_mode && !capturing) return run_graph(h, c, strat, s);
   return launch_all(h, c, strat, s);
 }
@@ -584,6 +660,9 @@ ftdx_status ftdx_init_herk(ftdx_handle h, int N, int K, int batch, void* stream)
   const HerkCall c{reinterpret_cast<const void*>(16), reinterpret_cast<void*>(16), N, K, batch,
                    FTDX_IN_INT4, FTDX_OUT_FP32, 1.f, 0.f};
   const Plan* p = nullptr;
+  Strategy strat;
+  if (!h->user_strategy && !stream_capturing(static_cast<cudaStream_t>(stream)))
+    return prepare_auto(h, c, static_cast<cudaStream_t>(stream), &strat);
   return prepare(h, c, static_cast<cudaStream_t>(stream), &p, use_pair(h, h->default_strategy));
 }
 
@@ -734,11 +813,14 @@ ftdx_status ftdx_herk_ftd(ftdx_handle h, const void* raw, void* C, const ftdx_ft
   cudaError_t e = cudaSetDevice(h->device);
   if (e != cudaSuccess) return cuda_fail(h, e, "cudaSetDevice");
   // strategy of the equivalent batch-first call (tuned entry if one exists)
-  Strategy strat = h->default_strategy;
+  Strategy strat = untuned_strategy(h, c);
   HerkCall plain = c;
   plain.ftd = nullptr;
   auto it = h->tuned.find(tune_key(h, plain));
-  if (it != h->tuned.end()) strat = it->second.st;
+  const bool tuned = it != h->tuned.end();
+  if (tuned) strat = it->second.st;
+  if (!tuned) st = prepare_auto(h, c, static_cast<cudaStream_t>(stream), &strat);
+  if (st != FTDX_OK) return st;
   return launch_all(h, c, strat, static_cast<cudaStream_t>(stream));
 }
 
@@ -782,7 +864,7 @@ ftdx_status ftdx_herk_kahan(ftdx_handle h, const void* A, void* sum, void* comp,
   // Read-modify-write of sum and compensation: no tuning sweep (it would
   // accumulate the same dump several times); direct stores only (the
   // single-CTA kernel, two-pass or with the promotion fused in).
-  Strategy strat = h->default_strategy;
+  Strategy strat = untuned_strategy(h, c);
   if (strat.store_mode != kStoreFused) strat.store_mode = 0;
   return launch_all(h, c, strat, static_cast<cudaStream_t>(stream));
 }
@@ -792,6 +874,7 @@ ftdx_status ftdx_set_split_k(ftdx_handle h, int splits) {
   if (splits < 1 || splits > 32)
     return fail(h, FTDX_ERR_INVALID_ARG, "set_split_k: splits must be 1..32 (got %d)", splits);
   h->default_strategy.splits = splits;
+  h->user_strategy = true;
   return FTDX_OK;
 }
 
@@ -814,6 +897,7 @@ ftdx_status ftdx_set_strategy(ftdx_handle h, int store_mode, int grid) {
       return fail(h, FTDX_ERR_UNSUPPORTED, "set_strategy: no CTA pair fits on this device");
   }
   h->default_strategy = Strategy{store_mode, grid, h->default_strategy.splits};
+  h->user_strategy = true;
   return FTDX_OK;
 }
 

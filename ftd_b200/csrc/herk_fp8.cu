@@ -1281,7 +1281,15 @@ __global__ void __launch_bounds__(256) split_reduce_kernel(const float2* __restr
     const int64_t c = x / P, p = x - c * P;
     const float2* w = ws + c * splits * P + p;
     float re = 0.f, im = 0.f;
-    for (int s = 0; s < splits; ++s) {
+    int s = 0;
+    for (; s + 4 <= splits; s += 4) {  // four loads in flight, summed in order
+      float2 v[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) v[u] = __ldcs(w + int64_t(s + u) * P);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) re += v[u].x, im += v[u].y;
+    }
+    for (; s < splits; ++s) {
       const float2 v = __ldcs(w + int64_t(s) * P);
       re += v.x;
       im += v.y;

@@ -8,6 +8,10 @@
 
 #include "ftdx.h"
 
+namespace ftdx {
+void clear_strategy(ftdx_handle h);  // herk_api.cu
+}
+
 namespace cutlass_gemm_api {
 
 struct CutlassComplexGemm::Impl {
@@ -47,8 +51,8 @@ struct CutlassComplexGemm::Impl {
       case HerkMode::ForceBaseline:
         if (ftdx_set_strategy(h, 2, 0) != FTDX_OK) ftdx_set_strategy(h, 0, 0);
         break;
-      case HerkMode::ForceDirect:
-      case HerkMode::Auto: ftdx_set_strategy(h, 0, 0); break;
+      case HerkMode::ForceDirect: ftdx_set_strategy(h, 0, 0); break;
+      case HerkMode::Auto: ftdx::clear_strategy(h); break;
     }
   }
 };

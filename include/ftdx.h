@@ -338,7 +338,11 @@ FTDX_API ftdx_status ftdx_lookup_tuned_compute(ftdx_handle h, int N, int K, int 
 FTDX_API ftdx_status ftdx_set_graph_mode(ftdx_handle h, int enable);
 FTDX_API int ftdx_graph_count(ftdx_handle h);
 
-/* Strategy for calls that are not tuned (tune = 0, or no cache entry):
+/* Strategy for calls that are not tuned (tune = 0, or no cache entry).  Until
+ * this or ftdx_set_split_k is called on a handle, the library picks by the
+ * call's sizes: the single-CTA kernel with direct stores, INT4 promotion
+ * apart or fused in (modes 0 and 16), and split-K where the tiles leave SMs
+ * idle.
  * store_mode 0 = direct stores, 1 = shared-memory staging + bulk copies,
  * 2 = CTA-pair kernel (one tcgen05 cta_group::2 MMA over two SMs per
  * 256 x 128 tile; uniform ftdx_herk calls, ftdx_herk_batched_v and

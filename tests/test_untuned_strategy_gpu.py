@@ -1,0 +1,93 @@
+"""Untuned calls on a handle that was given no strategy: the kernel (promotion
+apart or fused in) and the split of K follow the call's sizes.  Every shape is
+bit-exact against the oracle, through every entry point that takes the rule,
+and whatever a call needs under capture is there after init_herk or after one
+call of its shape."""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+from oracle import oracle  # noqa: E402
+
+from ftd_b200 import Correlator, tri_size  # noqa: E402
+from ftd_b200._lib import IN_INT4, OUT_FP16, OUT_FP32  # noqa: E402
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def device_bytes(qc, offset=0):
+    buf = torch.zeros(qc.size + offset, dtype=torch.uint8, device=DEV)
+    buf[offset:] = torch.from_numpy(qc.reshape(-1))
+    return buf[offset:]
+
+
+# one tile or several, below and above the splits' reach; K that the fused
+# kernel takes (multiples of 16) and that it does not; one k-block
+@pytest.mark.parametrize("N,K,B", [(1, 1, 1), (64, 8192, 1), (64, 8191, 1), (130, 12800, 3),
+                                   (256, 2048, 4), (257, 2050, 4), (128, 256, 32), (300, 128, 60),
+                                   (512, 4096, 1), (40, 30000, 5)])
+@pytest.mark.parametrize("offset", [0, 3])
+def test_bit_exact(N, K, B, offset):
+    qc = oracle.gaussian_qc(N + K, B, N, K)
+    ref = oracle.herk_qc(qc, N, K, B).astype(np.float32)
+    d = device_bytes(qc, offset)
+    C = torch.full((B, tri_size(N), 2), float("nan"), device=DEV)
+    C16 = torch.full((B, tri_size(N), 2), float("nan"), device=DEV, dtype=torch.float16)
+    S, comp = torch.zeros_like(C), torch.zeros_like(C)
+    with Correlator() as c:
+        c.herk(d, C, N, K, B, input=IN_INT4, output=OUT_FP32, tune=False)
+        c.herk(d, C16, N, K, B, input=IN_INT4, output=OUT_FP16, tune=False)
+        c.herk_kahan(d, S, comp, N, K, B, input=IN_INT4)
+        assert c.device_status() == 0
+    assert np.array_equal(C.cpu().numpy(), ref)
+    # integers beyond half's range: inf on both sides
+    with np.errstate(over="ignore"):
+        assert np.array_equal(C16.cpu().numpy(), ref.astype(np.float16))
+    assert np.array_equal(S.cpu().numpy(), ref)
+
+
+def test_alpha_beta_on_a_split_call():
+    N, K, B = 200, 8192, 2
+    qc = oracle.gaussian_qc(9, B, N, K)
+    R = oracle.herk_qc(qc, N, K, B)
+    old = torch.randn(B, tri_size(N), 2, device=DEV)
+    C = old.clone()
+    with Correlator() as c:
+        c.herk(device_bytes(qc), C, N, K, B, input=IN_INT4, output=OUT_FP32, alpha=0.5, beta=2.0,
+               tune=False)
+        assert c.device_status() == 0
+    np.testing.assert_allclose(C.double().cpu().numpy(),
+                               0.5 * R + 2.0 * old.double().cpu().numpy(), rtol=1e-6, atol=1e-3)
+
+
+@pytest.mark.parametrize("prepare", ["init", "call"])
+@pytest.mark.parametrize("offset", [0, 3])
+def test_capture(prepare, offset):
+    # after init_herk, or after one call on an aligned input, the shape can be
+    # captured on an input of any alignment, and with Kahan accumulation
+    N, K, B = 256, 8192, 2
+    qc = oracle.gaussian_qc(11, B, N, K)
+    ref = oracle.herk_qc(qc, N, K, B).astype(np.float32)
+    d = device_bytes(qc, offset)
+    C = torch.full((B, tri_size(N), 2), float("nan"), device=DEV)
+    S, comp = torch.zeros_like(C), torch.zeros_like(C)
+    s = torch.cuda.Stream()
+    with Correlator() as c:
+        if prepare == "init":
+            c.init_herk(N, K, B)
+        else:
+            c.herk(device_bytes(qc), C, N, K, B, input=IN_INT4, output=OUT_FP32, tune=False)
+            C.fill_(float("nan"))
+        torch.cuda.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=s):
+            c.herk(d, C, N, K, B, input=IN_INT4, output=OUT_FP32, tune=False, stream=s)
+            c.herk_kahan(d, S, comp, N, K, B, input=IN_INT4, stream=s)
+        S.zero_(), comp.zero_()
+        g.replay()
+        torch.cuda.synchronize()
+        assert np.array_equal(C.cpu().numpy(), ref)
+        assert np.array_equal(S.cpu().numpy(), ref)
+        assert c.device_status() == 0
+        del g
