@@ -126,6 +126,16 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* m, 
       : "memory");
 }
 
+// 4-D tiled load into shared memory, completing on mbarrier `bar`.
+__device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* m, int32_t x,
+                                            int32_t y, int32_t z, int32_t w, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes"
+      " [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(dst),
+      "l"(reinterpret_cast<uint64_t>(m)), "r"(x), "r"(y), "r"(z), "r"(w), "r"(bar)
+      : "memory");
+}
+
 // Bulk copy global -> shared (async proxy), completing on mbarrier `bar`.
 // Addresses 16-byte aligned, size a multiple of 16.
 __device__ __forceinline__ void bulk_load(uint32_t sdst, const void* gsrc, uint32_t bytes,
@@ -417,6 +427,19 @@ __device__ __forceinline__ uint64_t sdesc_sw128_kmajor(uint32_t saddr) {
   return d;
 }
 
+// The same for an MN-major operand: rows of 64 16-bit MN elements (128 bytes),
+// one per k, 8 k rows every 1024 bytes, and `chunk` bytes from one 64-element
+// MN chunk to the next.
+__device__ __forceinline__ uint64_t sdesc_sw128_mnmajor(uint32_t saddr, uint32_t chunk) {
+  uint64_t d = 0;
+  d |= static_cast<uint64_t>((saddr & 0x3FFFFu) >> 4);  // start address  [0,14)
+  d |= static_cast<uint64_t>(chunk >> 4) << 16;          // LBO: next MN chunk
+  d |= static_cast<uint64_t>(1024 >> 4) << 32;           // SBO: next 8 k rows
+  d |= static_cast<uint64_t>(1) << 46;                   // descriptor version (sm100)
+  d |= static_cast<uint64_t>(2) << 61;                   // layout: SWIZZLE_128B
+  return d;
+}
+
 // Descriptor of an unswizzled K-major shared-memory source: rows of 16 bytes
 // back to back, 8-row core matrices `sbo` bytes apart (tcgen05.cp sources).
 __device__ __forceinline__ uint64_t sdesc_none_kmajor(uint32_t saddr, uint32_t sbo) {
@@ -442,6 +465,8 @@ __device__ __forceinline__ void tmem_cp_32x128b_warpx4(uint32_t taddr, uint64_t 
 //   neg_a: negate A (valid for kind::f16 and kind::f8f6f4).
 // kind::f8f6f4 operand formats (instruction descriptor a/b format fields).
 constexpr uint32_t kFmtE4M3 = 0, kFmtE3M2 = 4;
+// instruction descriptor bits: A / B is MN-major (16-bit operand types)
+constexpr uint32_t kIdescAMnMajor = 1u << 15, kIdescBMnMajor = 1u << 16;
 // kind::i8: signed 8-bit A and B, S32 accumulator, K-major.
 __host__ __device__ constexpr uint32_t idesc_s32acc_s8(uint32_t M, uint32_t N) {
   return (2u << 4)                 // D format: S32
