@@ -231,8 +231,21 @@ Strategy auto_strategy(const ftdx_context& h, int N, int K, int batch, bool fuse
   return best;
 }
 
+// NVFP4: the CTA pair from four rounds of its tiles on, where the operand
+// bytes it saves per tile outweigh its coarser tiles, and from four k-blocks
+// on, where the loads and not the stores set the pace.  Single CTA / pair, us:
+// 4096 inputs x 1024 x 16: 995 / 926; 2048 x 1024 x 8 (9 rounds): 204 / 194;
+// 1500 x 1000 x 4 (3 rounds): 78 / 78; 1024 x 512 x 4: 39 / 45;
+// 4096 x 128 x 4 (one k-block): 111 / 125.
+Strategy fp4_strategy(int N, int K, int batch) {
+  const int64_t nj = (N + 255) / 256, tiles = nj * (nj + 1) * 8 / 7 * batch;  // ~ of 256 x 112
+  const int pairs = nvfp4_pair_limit();
+  return Strategy{pairs >= 1 && tiles >= 4 * pairs && nvfp4_kblocks(K) >= 4 ? 2 : 0, 0};
+}
+
 Strategy untuned_strategy(ftdx_handle h, const HerkCall& c) {
-  if (h->user_strategy || is_fp4(c)) return h->default_strategy;
+  if (h->user_strategy) return h->default_strategy;
+  if (is_fp4(c)) return fp4_strategy(c.N, c.K, c.batch);
   return auto_strategy(*h, c.N, c.K, c.batch, fused_ok(c), !c.comp && c.out_format == 0);
 }
 

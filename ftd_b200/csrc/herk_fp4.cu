@@ -368,12 +368,24 @@ __global__ void __launch_bounds__(1024) nvfp4_order_kernel(const uint32_t* __res
 // Pass 3, one warp per input row: the E2M1 operands and UE4M3 scale atoms in
 // the channel's time order (lane l: blocks l, l + 32, ...), with the lo
 // residual in the blocks of the trailing chans[c].pad k-blocks.
-__global__ void __launch_bounds__(256, 4) nvfp4_quant_kernel(
+// A lane's block is 64 bytes of the row, so lanes that load their blocks
+// themselves ask for 32 sectors with every load, eight loads per block where
+// the time order is permuted: the L1 was busy 86% of the time (241 us for 16
+// channels of 4096 x 1024, 34% of DRAM).  kStaged: the warp copies the row to
+// shared memory in consecutive 16-byte loads, one float2 of padding per block
+// (lanes 72 bytes apart: no bank conflict), and the lanes read it there.
+// Rows longer than kStageSamples are read in place.
+// There: 241 -> 210 us, the same codes.
+constexpr int kStageSamples = 1024;
+__host__ __device__ constexpr size_t stage_bytes_per_row(int K) { return size_t((K + 7) / 8) * 9 * sizeof(float2); }
+template <bool kStaged>
+__global__ void __launch_bounds__(256, kStaged ? 3 : 4) nvfp4_quant_kernel(
     const float2* __restrict__ a, const int32_t* __restrict__ src,
     const int32_t* __restrict__ nflag, const ChanDesc* __restrict__ chans,
     const float* __restrict__ rscale, uint8_t* __restrict__ z, uint8_t* __restrict__ sfa,
     uint8_t* __restrict__ sfb, int64_t rows, int K, int kp, int pitch, SfGeom sg) {
   const int lane = threadIdx.x & 31;
+  extern __shared__ __align__(16) uint8_t stage_smem[];  // kStaged: a row per warp
   const int blocks_per_row = pitch / 8;  // 8 bytes of E2M1 per block
   const bool vec = (K & 1) == 0 && (reinterpret_cast<uintptr_t>(a) & 15) == 0;
   for (int64_t r = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; r < rows;
@@ -385,25 +397,81 @@ __global__ void __launch_bounds__(256, 4) nvfp4_quant_kernel(
     const int lo_from = (kp / 128 - chans[c].pad) * 16;  // first block with a residual
     const int32_t* sc = src + int64_t(c) * kp;
     const Fp4RowOut o = fp4_row_out(r, c, w, z, sfa, sfb, pitch, sg);
-    for (int b = lane; b < blocks_per_row; b += 32) {
-      const int t0 = 8 * b;
-      float x[16];
-      if (!permuted && vec && t0 + 8 <= K) {
-        const float4* p4 = reinterpret_cast<const float4*>(p + t0);
+    if constexpr (kStaged) {
+      float2* row = reinterpret_cast<float2*>(
+          stage_smem + (threadIdx.x >> 5) * stage_bytes_per_row(K));
+      __syncwarp();  // the previous row has been read
+      if (vec) {
+        const float4* p4 = reinterpret_cast<const float4*>(p);
+        for (int t2 = lane; t2 < K / 2; t2 += 128) {  // four 16-byte loads in flight per lane
+          float4 v[4];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const float4 v = __ldg(p4 + q);
-          x[4 * q] = v.x, x[4 * q + 1] = v.y, x[4 * q + 2] = v.z, x[4 * q + 3] = v.w;
+          for (int u = 0; u < 4; ++u)
+            if (t2 + 32 * u < K / 2) v[u] = __ldg(p4 + t2 + 32 * u);
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const int t = 2 * (t2 + 32 * u);
+            if (t < K) {
+              row[t + (t >> 3)] = make_float2(v[u].x, v[u].y);
+              row[t + (t >> 3) + 1] = make_float2(v[u].z, v[u].w);
+            }
+          }
         }
       } else {
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          const int t = permuted ? (t0 + q < kp ? __ldg(sc + t0 + q) : -1) : (t0 + q < K ? t0 + q : -1);
-          const float2 v = t >= 0 ? __ldg(p + t) : make_float2(0.f, 0.f);
-          x[2 * q] = v.x, x[2 * q + 1] = v.y;
-        }
+        for (int t = lane; t < K; t += 32) row[t + (t >> 3)] = __ldg(p + t);
       }
-      nvfp4_block(x, g, b, o, b >= lo_from);
+      __syncwarp();
+      for (int b = lane; b < blocks_per_row; b += 32) {
+        const int t0 = 8 * b;
+        float x[16];
+        if (!permuted && t0 + 8 <= K) {
+#pragma unroll
+          for (int q = 0; q < 8; ++q) {
+            const float2 v = row[9 * b + q];
+            x[2 * q] = v.x, x[2 * q + 1] = v.y;
+          }
+        } else {
+          // positions past K have source -1 (t0 < kp: the order covers the padding)
+          int src8[8];
+          if (permuted) {
+            const int4 s0 = __ldg(reinterpret_cast<const int4*>(sc + t0));
+            const int4 s1 = __ldg(reinterpret_cast<const int4*>(sc + t0) + 1);
+            src8[0] = s0.x, src8[1] = s0.y, src8[2] = s0.z, src8[3] = s0.w;
+            src8[4] = s1.x, src8[5] = s1.y, src8[6] = s1.z, src8[7] = s1.w;
+          } else {
+#pragma unroll
+            for (int q = 0; q < 8; ++q) src8[q] = t0 + q < K ? t0 + q : -1;
+          }
+#pragma unroll
+          for (int q = 0; q < 8; ++q) {
+            const int t = src8[q];
+            const float2 v = t >= 0 ? row[t + (t >> 3)] : make_float2(0.f, 0.f);
+            x[2 * q] = v.x, x[2 * q + 1] = v.y;
+          }
+        }
+        nvfp4_block(x, g, b, o, b >= lo_from);
+      }
+    } else {
+      for (int b = lane; b < blocks_per_row; b += 32) {
+        const int t0 = 8 * b;
+        float x[16];
+        if (!permuted && vec && t0 + 8 <= K) {
+          const float4* p4 = reinterpret_cast<const float4*>(p + t0);
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const float4 v = __ldg(p4 + q);
+            x[4 * q] = v.x, x[4 * q + 1] = v.y, x[4 * q + 2] = v.z, x[4 * q + 3] = v.w;
+          }
+        } else {
+#pragma unroll
+          for (int q = 0; q < 8; ++q) {
+            const int t = permuted ? (t0 + q < kp ? __ldg(sc + t0 + q) : -1) : (t0 + q < K ? t0 + q : -1);
+            const float2 v = t >= 0 ? __ldg(p + t) : make_float2(0.f, 0.f);
+            x[2 * q] = v.x, x[2 * q + 1] = v.y;
+          }
+        }
+        nvfp4_block(x, g, b, o, b >= lo_from);
+      }
     }
   }
 }
@@ -1045,14 +1113,10 @@ cudaError_t launch_nvfp4(const void* A, int64_t rows, int K, int n, int batch, u
   uint32_t* flags = reinterpret_cast<uint32_t*>(sfb + w.sfb_bytes + 2 * w.pw_bytes);
   int32_t* nflag = reinterpret_cast<int32_t*>(reinterpret_cast<uint8_t*>(flags) + w.flag_bytes);
   int32_t* src = reinterpret_cast<int32_t*>(reinterpret_cast<uint8_t*>(nflag) + w.nflag_bytes);
-  // rows of a partial group get no scales from the quantiser: zero them
-  // (their products land only in outputs the epilogue skips)
   cudaError_t e;
   if (phases & 1) {  // the quantiser passes
-    if (n % (pair ? k4pJ : 128) != 0 || (2 * n) % w.sg.gbrows != 0) {
-      e = cudaMemsetAsync(sfa, 0, size_t(w.sfa_bytes + w.sfb_bytes), s);
-      if (e != cudaSuccess) return e;
-    }
+    // rows of a partial group get no scales: whatever they hold reaches only
+    // accumulator rows and columns past n, which the epilogue skips
     const int rfi = split ? 0 : 1;
     if (rfi) {
       e = cudaMemsetAsync(flags, 0, size_t(w.flag_bytes), s);
@@ -1068,9 +1132,19 @@ cudaError_t launch_nvfp4(const void* A, int64_t rows, int K, int n, int batch, u
                                                         const_cast<ChanDesc*>(chans), K,
                                                         int(w.kp), w.fwords, split);
     // E2M1 operands and UE4M3 scale atoms
-    nvfp4_quant_kernel<<<unsigned(blocks), 256, 0, s>>>(static_cast<const float2*>(A), src, nflag,
-                                                        chans, rscale, z, sfa, sfb, rows, K,
-                                                        int(w.kp), int(pitch), w.sg);
+    auto quantise = [&](auto kernel, size_t smem) {
+      kernel<<<unsigned(blocks), 256, smem, s>>>(static_cast<const float2*>(A), src, nflag, chans,
+                                                 rscale, z, sfa, sfb, rows, K, int(w.kp),
+                                                 int(pitch), w.sg);
+    };
+    if (K <= kStageSamples) {
+      e = ensure_smem_limit(reinterpret_cast<const void*>(nvfp4_quant_kernel<true>),
+                            8 * stage_bytes_per_row(kStageSamples));
+      if (e != cudaSuccess) return e;
+      quantise(nvfp4_quant_kernel<true>, 8 * stage_bytes_per_row(K));
+    } else {
+      quantise(nvfp4_quant_kernel<false>, 0);
+    }
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }
