@@ -7,8 +7,9 @@
 //  * herk_fp8_tc_kernel: persistent, warp-specialised tcgen05 HERK.  Each CTA
 //    walks a list of lower-triangle tiles (128 column antennas j x 128 row
 //    antennas i).  TMA feeds a 3-stage ring of four 128 x 128-byte planes
-//    (Re_j, Im_j, Re_i, Im_i); one thread issues four tcgen05.mma kind::f8f6f4
-//    (M = N = 128, K = 32) per k-step into a Re and an Im accumulator in TMEM
+//    (Re_j, Im_j, Re_i, Im_i); one thread issues three tcgen05.mma kind::f8f6f4
+//    (M = 128, K = 32; N = 256 once, 128 twice) per k-step into a Re and an Im
+//    accumulator in TMEM
 //    (double-buffered); four epilogue warps drain the other accumulator with
 //    tcgen05.ld and store the packed lower triangle directly.  TMEM lane j
 //    holds R_ij for consecutive i in consecutive columns, so a warp's 32
@@ -504,6 +505,14 @@ __global__ void __launch_bounds__(kFused ? kFusedThreads : kHerkThreads, 1)
       const uint32_t fmt = args.fp6 ? kFmtE3M2 : kFmtE4M3;
       const uint32_t idesc = idesc_f32acc(fmt, fmt, kTile, kTile);
       const uint32_t idesc_neg = idesc_f32acc(fmt, fmt, kTile, kTile, 1);
+      // Re_i and Im_i lie back to back: 256 rows of one B operand, into the Re
+      // and the Im columns of the accumulator.  Re_j is read once for both:
+      // shared memory (operands, TMA writes, stores) sets the tensor pipe's
+      // pace, 1690 clocks per k-block with four MMAs of N = 128, 1626 so (1024
+      // without the other traffic; 4096 inputs, K = 1024, 16 channels: 459 ->
+      // 449 us).  A ring of seven half stages in place of three stages did not
+      // pay: 3% slower where the MMAs dominate.
+      const uint32_t idesc_wide = idesc_f32acc(fmt, fmt, kTile, 2 * kTile);
       int stage = 0;
       uint32_t phase = 0;
       int acc = 0;
@@ -542,8 +551,8 @@ __global__ void __launch_bounds__(kFused ? kFusedThreads : kHerkThreads, 1)
             const uint64_t dbre = sdesc_sw128_kmajor(bre + 32 * s);
             const uint64_t dbim = sdesc_sw128_kmajor(bim + 32 * s);
             const uint32_t first = (kb | s) != 0;
-            mma_f8f6f4(d_re, dare, dbre, idesc, first);     // Re += Re_j Re_i
-            mma_f8f6f4(d_im, dare, dbim, idesc, first);     // Im += Re_j Im_i
+            // Re += Re_j Re_i and Im += Re_j Im_i
+            mma_f8f6f4(d_re, dare, dbre, idesc_wide, first);
             mma_f8f6f4(d_re, daim, dbim, idesc, 1);         // Re += Im_j Im_i
             mma_f8f6f4(d_im, daim, dbre, idesc_neg, 1);     // Im -= Im_j Re_i
           }
