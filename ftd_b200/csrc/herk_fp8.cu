@@ -333,19 +333,31 @@ __device__ __forceinline__ void store_chunk(Out2* p, float2* pc, int i0, int j, 
 // byte each) into a ring of kRawStages, and four converter warps (warps 10-13)
 // turn each into the E4M3 Re / Im planes of an operand stage in the 128-byte
 // swizzled layout the TMA would have written, then release it to the MMA warp.
-template <typename OutT, bool kFused>
+//
+// kSplit (hi + lo operands, hi hi^H + hi lo^H + lo hi^H): a k-block's four
+// units -- hi_j, hi_i, lo_i, lo_j; on the diagonal hi and lo -- are loaded once
+// for its three products.  Taking the products one after the other over all of
+// K loaded hi_j and hi_i twice: 192 KB per k-block instead of 128 KB, written
+// into the shared memory whose traffic sets the MMAs' pace.  A ring of seven
+// units holds one k-block and most of the next; hi_j and lo_i are free after
+// the second product, so the loads of the next k-block's last units have the
+// third and the next two to arrive.  4096 inputs, K = 1024, 16 channels: 1722
+// -> 1566 us a call.
+template <typename OutT, bool kFused, bool kSplit>
 __global__ void __launch_bounds__(kFused ? kFusedThreads : kHerkThreads, 1)
     herk_fp8_tc_kernel(const __grid_constant__ CUtensorMap tmZ, const HerkArgs args) {
-  constexpr int kOpStages = kFused ? kFusedStages : kStages;
+  static_assert(!(kFused && kSplit), "split operands come from the float promotion");
+  constexpr int kOpStages = kFused ? kFusedStages : (kSplit ? kSplitUnits : kStages);
+  constexpr int kOpBytes = kSplit ? kUnitBytes : kStageBytes;  // of one operand stage
   constexpr int kBarCount = 2 * kOpStages + 5 + (kFused ? 2 * kRawStages : 0);
   extern __shared__ uint8_t smem_dyn[];
   // 128 B swizzled operand tiles must start on 1024 B boundaries of the
   // shared window.
   uint8_t* smem = smem_dyn + ((1024u - (smem_u32(smem_dyn) & 1023u)) & 1023u);
   // epilogue staging (kStgBytes); with kFused the raw QC ring instead
-  uint8_t* stg_base = smem + kOpStages * kStageBytes;
+  uint8_t* stg_base = smem + kOpStages * kOpBytes;
   uint64_t* bars = reinterpret_cast<uint64_t*>(
-      stg_base + (kFused ? size_t(kRawStages) * kRawStageBytes : size_t(kStgBytes)));
+      stg_base + (kFused ? size_t(kRawStages) * kRawStageBytes : (kSplit ? 0 : size_t(kStgBytes))));
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + kBarCount);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
@@ -360,11 +372,11 @@ __global__ void __launch_bounds__(kFused ? kFusedThreads : kHerkThreads, 1)
   auto rfull_bar = [&](int r) { return bar0 + 8u * (2 * kOpStages + 5 + r); };
   auto rempty_bar = [&](int r) { return bar0 + 8u * (2 * kOpStages + 5 + kRawStages + r); };
   auto raw_addr = [&](int r) {
-    return smem0 + uint32_t(kOpStages * kStageBytes + r * kRawStageBytes);
+    return smem0 + uint32_t(kOpStages * kOpBytes + r * kRawStageBytes);
   };
-  // plane p of stage s: 0 = Re_j, 1 = Im_j, 2 = Re_i, 3 = Im_i
+  // plane p of stage s: 0 = Re_j, 1 = Im_j, 2 = Re_i, 3 = Im_i (kSplit: 0 = Re, 1 = Im)
   auto plane_addr = [&](int s, int p) {
-    return smem0 + uint32_t(s * kStageBytes + p * kPlaneBytes);
+    return smem0 + uint32_t(s * kOpBytes + p * kPlaneBytes);
   };
 
   const int warp = threadIdx.x >> 5;
@@ -457,31 +469,50 @@ __global__ void __launch_bounds__(kFused ? kFusedThreads : kHerkThreads, 1)
         const int32_t rowJ = int32_t(cd.row0 + int64_t(swap ? td.ti : td.tj) * kTile);
         const int32_t rowI = int32_t(cd.row0 + int64_t(swap ? td.tj : td.ti) * kTile);
         const bool diag = td.ti == td.tj;  // i block == j block: load it once
-        const int nkb = cd.kblocks * args.nseg;
-        for (int kb = 0; kb < nkb; ++kb) {
-          if (!mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag)) {
-            atomicOr(args.status, kStatusTimeoutProducer);
-            ok = false;
-            break;
+        if constexpr (kSplit) {
+          const int32_t lo = args.seg_b[1];  // k-blocks from the hi to the lo columns
+          for (int kb = 0; kb < cd.kblocks && ok; ++kb) {
+            const int32_t x_hi = (cd.kb0 + kb) * kStageK, x_lo = x_hi + lo * kStageK;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {  // hi_j, hi_i, lo_i, lo_j
+              if (diag && (u == 1 || u == 2)) continue;
+              if (!mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag)) {
+                atomicOr(args.status, kStatusTimeoutProducer);
+                ok = false;
+                break;
+              }
+              const int32_t x = u < 2 ? x_hi : x_lo, row = (u == 0 || u == 3) ? rowJ : rowI;
+              mbar_arrive_expect_tx(full_bar(stage), kUnitBytes);
+              tma_load_3d(plane_addr(stage, 0), &tmZ, x, row, 0, full_bar(stage));
+              tma_load_3d(plane_addr(stage, 1), &tmZ, x, row, 1, full_bar(stage));
+              ++issued;
+              if (++stage == kOpStages) {
+                stage = 0;
+                phase ^= 1u;
+              }
+            }
           }
-          const int seg = kb / cd.kblocks;
-          const int kk = kb - seg * cd.kblocks;
-          const int sa = seg == 0 ? args.seg_a[0] : (seg == 1 ? args.seg_a[1] : args.seg_a[2]);
-          const int sb = seg == 0 ? args.seg_b[0] : (seg == 1 ? args.seg_b[1] : args.seg_b[2]);
-          const int32_t kA = (sa + cd.kb0 + kk) * kStageK, kB = (sb + cd.kb0 + kk) * kStageK;
-          const bool share = diag && sa == sb;
-          const uint32_t bytes = share ? 2 * kPlaneBytes : kStageBytes;  // FP8 planes
-          mbar_arrive_expect_tx(full_bar(stage), args.fp6 ? bytes / 4 * 3 : bytes);
-          tma_load_3d(plane_addr(stage, 0), &tmZ, kA, rowJ, 0, full_bar(stage));
-          tma_load_3d(plane_addr(stage, 1), &tmZ, kA, rowJ, 1, full_bar(stage));
-          if (!share) {
-            tma_load_3d(plane_addr(stage, 2), &tmZ, kB, rowI, 0, full_bar(stage));
-            tma_load_3d(plane_addr(stage, 3), &tmZ, kB, rowI, 1, full_bar(stage));
-          }
-          ++issued;
-          if (++stage == kStages) {
-            stage = 0;
-            phase ^= 1u;
+        } else {
+          for (int kb = 0; kb < cd.kblocks; ++kb) {
+            if (!mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag)) {
+              atomicOr(args.status, kStatusTimeoutProducer);
+              ok = false;
+              break;
+            }
+            const int32_t x = (cd.kb0 + kb) * kStageK;
+            const uint32_t bytes = diag ? 2 * kPlaneBytes : kStageBytes;  // FP8 planes
+            mbar_arrive_expect_tx(full_bar(stage), args.fp6 ? bytes / 4 * 3 : bytes);
+            tma_load_3d(plane_addr(stage, 0), &tmZ, x, rowJ, 0, full_bar(stage));
+            tma_load_3d(plane_addr(stage, 1), &tmZ, x, rowJ, 1, full_bar(stage));
+            if (!diag) {
+              tma_load_3d(plane_addr(stage, 2), &tmZ, x, rowI, 0, full_bar(stage));
+              tma_load_3d(plane_addr(stage, 3), &tmZ, x, rowI, 1, full_bar(stage));
+            }
+            ++issued;
+            if (++stage == kOpStages) {
+              stage = 0;
+              phase ^= 1u;
+            }
           }
         }
       }
@@ -489,9 +520,9 @@ __global__ void __launch_bounds__(kFused ? kFusedThreads : kHerkThreads, 1)
         // Let every load still in flight land before the CTA exits.
         int s = stage;
         uint32_t ph = phase;
-        for (int n = 0; n < kStages && n < issued; ++n) {
+        for (int n = 0; n < kOpStages && n < issued; ++n) {
           if (--s < 0) {
-            s = kStages - 1;
+            s = kOpStages - 1;
             ph ^= 1u;
           }
           volatile int never = 0;
@@ -530,32 +561,65 @@ __global__ void __launch_bounds__(kFused ? kFusedThreads : kHerkThreads, 1)
         tc_fence_after();
         const uint32_t d_re = tmem_base + uint32_t(acc * kAccCols);
         const uint32_t d_im = d_re + uint32_t(kTile);
-        const int nkb = cd.kblocks * args.nseg;
-        for (int kb = 0; kb < nkb; ++kb) {
+        // the four products of a j block (Re, then Im plane at aj) and an i block (bi)
+        auto product = [&](uint32_t aj, uint32_t bi, bool first) {
+#pragma unroll
+          for (int s = 0; s < kStageK / 32; ++s) {
+            const uint64_t dare = sdesc_sw128_kmajor(aj + 32 * s);
+            const uint64_t daim = sdesc_sw128_kmajor(aj + kPlaneBytes + 32 * s);
+            const uint64_t dbre = sdesc_sw128_kmajor(bi + 32 * s);
+            const uint64_t dbim = sdesc_sw128_kmajor(bi + kPlaneBytes + 32 * s);
+            // Re += Re_j Re_i and Im += Re_j Im_i
+            mma_f8f6f4(d_re, dare, dbre, idesc_wide, !first || s != 0);
+            mma_f8f6f4(d_re, daim, dbim, idesc, 1);      // Re += Im_j Im_i
+            mma_f8f6f4(d_im, daim, dbre, idesc_neg, 1);  // Im -= Im_j Re_i
+          }
+        };
+        if constexpr (kSplit) {
+          // waits for the ring's next unit and returns its stage (-1: gave up)
+          auto next_unit = [&]() {
+            if (!mbar_wait(full_bar(stage), phase, abort_flag)) {
+              atomicOr(args.status, kStatusTimeoutMma);
+              ok = false;
+              return -1;
+            }
+            tc_fence_after();
+            const int u = stage;
+            if (++stage == kOpStages) {
+              stage = 0;
+              phase ^= 1u;
+            }
+            return u;
+          };
+          for (int kb = 0; kb < cd.kblocks; ++kb) {
+            const int hj = next_unit();
+            if (hj < 0) break;
+            const int hi = diag ? hj : next_unit();
+            if (hi < 0) break;
+            product(plane_addr(hj, 0), plane_addr(hi, 0), kb == 0);
+            const int li = next_unit();
+            if (li < 0) break;
+            product(plane_addr(hj, 0), plane_addr(li, 0), false);
+            int lj = li;
+            if (!diag) {
+              mma_commit(empty_bar(hj));
+              mma_commit(empty_bar(li));
+              lj = next_unit();
+              if (lj < 0) break;
+            }
+            product(plane_addr(lj, 0), plane_addr(hi, 0), false);
+            mma_commit(empty_bar(hi));
+            mma_commit(empty_bar(lj));
+          }
+        }
+        for (int kb = 0; !kSplit && kb < cd.kblocks; ++kb) {
           if (!mbar_wait(full_bar(stage), phase, abort_flag)) {
             atomicOr(args.status, kStatusTimeoutMma);
             ok = false;
             break;
           }
           tc_fence_after();
-          const int seg = kb / cd.kblocks;
-          const int sa = seg == 0 ? args.seg_a[0] : (seg == 1 ? args.seg_a[1] : args.seg_a[2]);
-          const int sb = seg == 0 ? args.seg_b[0] : (seg == 1 ? args.seg_b[1] : args.seg_b[2]);
-          const int pb = (diag && sa == sb) ? 0 : 2;  // planes holding the i block
-          const uint32_t are = plane_addr(stage, 0), aim = plane_addr(stage, 1);
-          const uint32_t bre = plane_addr(stage, pb), bim = plane_addr(stage, pb + 1);
-#pragma unroll
-          for (int s = 0; s < kStageK / 32; ++s) {
-            const uint64_t dare = sdesc_sw128_kmajor(are + 32 * s);
-            const uint64_t daim = sdesc_sw128_kmajor(aim + 32 * s);
-            const uint64_t dbre = sdesc_sw128_kmajor(bre + 32 * s);
-            const uint64_t dbim = sdesc_sw128_kmajor(bim + 32 * s);
-            const uint32_t first = (kb | s) != 0;
-            // Re += Re_j Re_i and Im += Re_j Im_i
-            mma_f8f6f4(d_re, dare, dbre, idesc_wide, first);
-            mma_f8f6f4(d_re, daim, dbim, idesc, 1);         // Re += Im_j Im_i
-            mma_f8f6f4(d_im, daim, dbre, idesc_neg, 1);     // Im -= Im_j Re_i
-          }
+          product(plane_addr(stage, 0), plane_addr(stage, diag ? 0 : 2), kb == 0);
           mma_commit(empty_bar(stage));
           if (++stage == kOpStages) {
             stage = 0;
@@ -608,7 +672,7 @@ __global__ void __launch_bounds__(kFused ? kFusedThreads : kHerkThreads, 1)
       const int ib = int(td.ti) * kTile;
       const uint32_t tb = tmem_base + (uint32_t(q * 32) << 16) + uint32_t(acc * kAccCols);
       Out2* outc = cd.out_ptr ? reinterpret_cast<Out2*>(cd.out_ptr) : out + cd.out0;
-      if (!kFused && kBulkOut && args.bulk_store && plain && td.ti != td.tj && ib + kTile <= n) {
+      if (!kFused && !kSplit && kBulkOut && args.bulk_store && plain && td.ti != td.tj && ib + kTile <= n) {
         // Interior tile: stage kStgRows row segments (128 consecutive packed
         // elements each) in shared memory, then one bulk copy per row.  A
         // row whose global start is 8 mod 16 keeps that phase in shared
@@ -1166,7 +1230,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kHerkThreads, 1)
 // fewer blocks start) and at least one.  One fixed size of 8192 pieces gave
 // 32 channels of 128 x 256 eight blocks (21.9 us of promotion) and 16 of
 // 1024 x 1024 FP16 samples 256 (24.6 us).
-static int rows_per_block(int64_t rows, int chunks) {
+int promotion_rows_per_block(int64_t rows, int chunks) {
   constexpr int64_t kBlocks = 8 * 148;
   const int64_t most = 8192 / chunks, least = (256 + chunks - 1) / chunks;
   int64_t r = rows / kBlocks;
@@ -1177,7 +1241,7 @@ static int rows_per_block(int64_t rows, int chunks) {
 
 cudaError_t launch_qc_to_planes(const uint8_t* qc, uint8_t* z, int64_t rows, int K, int Kp,
                                 cudaStream_t s, bool neg_plane) {
-  const int rpb = rows_per_block(rows, Kp >> 4);
+  const int rpb = promotion_rows_per_block(rows, Kp >> 4);
   const int64_t blocks = (rows + rpb - 1) / rpb;
   qc_to_planes_kernel<<<unsigned(blocks), 256, 0, s>>>(qc, z, rows, K, Kp, rpb, neg_plane ? 1 : 0);
   return cudaGetLastError();
@@ -1185,7 +1249,7 @@ cudaError_t launch_qc_to_planes(const uint8_t* qc, uint8_t* z, int64_t rows, int
 
 cudaError_t launch_qc_to_planes_s8(const uint8_t* qc, uint8_t* z, int64_t rows, int K, int Kp,
                                    cudaStream_t s, bool neg_plane) {
-  const int rpb = rows_per_block(rows, Kp >> 4);
+  const int rpb = promotion_rows_per_block(rows, Kp >> 4);
   const int64_t blocks = (rows + rpb - 1) / rpb;
   qc_to_planes_s8_kernel<<<unsigned(blocks), 256, 0, s>>>(qc, z, rows, K, Kp, rpb,
                                                            neg_plane ? 1 : 0);
@@ -1194,7 +1258,7 @@ cudaError_t launch_qc_to_planes_s8(const uint8_t* qc, uint8_t* z, int64_t rows, 
 
 cudaError_t launch_qc_to_planes6(const uint8_t* qc, uint8_t* z, int64_t rows, int K, int Kp,
                                  cudaStream_t s, bool neg_plane) {
-  const int rpb = rows_per_block(rows, Kp >> 4);
+  const int rpb = promotion_rows_per_block(rows, Kp >> 4);
   const int64_t blocks = (rows + rpb - 1) / rpb;
   qc_to_planes6_kernel<<<unsigned(blocks), 256, 0, s>>>(qc, z, rows, K, Kp, rpb,
                                                          neg_plane ? 1 : 0);
@@ -1212,7 +1276,7 @@ cudaError_t launch_negate_plane(uint8_t* z, int64_t plane_bytes, int sm_count, c
 
 cudaError_t launch_fp16_to_planes(const void* a16, uint8_t* z, int64_t rows, int K, int Kp,
                                   cudaStream_t s) {
-  const int rpb = rows_per_block(rows, Kp >> 3);
+  const int rpb = promotion_rows_per_block(rows, Kp >> 3);
   const int64_t blocks = (rows + rpb - 1) / rpb;
   fp16_to_planes_kernel<<<unsigned(blocks), 256, 0, s>>>(
       static_cast<const __half2*>(a16), z, rows, K, Kp, rpb,
@@ -1222,21 +1286,21 @@ cudaError_t launch_fp16_to_planes(const void* a16, uint8_t* z, int64_t rows, int
 
 cudaError_t launch_gather_qc_to_planes(const GatherDesc* g, int nch, int max_n, uint8_t* z,
                                        int64_t total_rows, int Kp, cudaStream_t s, int neg_plane) {
-  const int rpb = rows_per_block(total_rows, Kp >> 4);
+  const int rpb = promotion_rows_per_block(total_rows, Kp >> 4);
   const dim3 grid(unsigned((max_n + rpb - 1) / rpb), unsigned(nch));
   gather_qc_to_planes_kernel<<<grid, 256, 0, s>>>(g, z, total_rows, Kp, rpb, neg_plane);
   return cudaGetLastError();
 }
 
-template <typename OutT, bool kFused>
+template <typename OutT, bool kFused, bool kSplit>
 static cudaError_t launch_herk_t(const CUtensorMap& tmZ, const HerkArgs& a, int grid,
                                  cudaStream_t s) {
-  constexpr size_t smem = kFused ? kFusedSmem : kHerkSmem;
+  constexpr size_t smem = kFused ? kFusedSmem : (kSplit ? kSplitSmem : kHerkSmem);
   constexpr int threads = kFused ? kFusedThreads : kHerkThreads;
-  cudaError_t e =
-      ensure_smem_limit(reinterpret_cast<const void*>(herk_fp8_tc_kernel<OutT, kFused>), smem);
+  cudaError_t e = ensure_smem_limit(
+      reinterpret_cast<const void*>(herk_fp8_tc_kernel<OutT, kFused, kSplit>), smem);
   if (e != cudaSuccess) return e;
-  herk_fp8_tc_kernel<OutT, kFused><<<grid, threads, smem, s>>>(tmZ, a);
+  herk_fp8_tc_kernel<OutT, kFused, kSplit><<<grid, threads, smem, s>>>(tmZ, a);
   return cudaGetLastError();
 }
 
@@ -1332,16 +1396,21 @@ cudaError_t launch_split_reduce(const float2* ws, void* out, int out_fp16, int64
 }
 
 cudaError_t launch_herk_fp8(const CUtensorMap& tmZ, const HerkArgs& a, int grid, cudaStream_t s) {
-  return a.out_fp16 ? launch_herk_t<__half, false>(tmZ, a, grid, s)
-                    : launch_herk_t<float, false>(tmZ, a, grid, s);
+  if (a.nseg != 1) {  // (hi, hi), (hi, lo), (lo, hi)
+    if (a.nseg != 3 || a.out_format != 0 || a.fp6) return cudaErrorInvalidValue;
+    return a.out_fp16 ? launch_herk_t<__half, false, true>(tmZ, a, grid, s)
+                      : launch_herk_t<float, false, true>(tmZ, a, grid, s);
+  }
+  return a.out_fp16 ? launch_herk_t<__half, false, false>(tmZ, a, grid, s)
+                    : launch_herk_t<float, false, false>(tmZ, a, grid, s);
 }
 
 cudaError_t launch_herk_fp8_fused(const CUtensorMap& tmQ, const HerkArgs& a, int grid,
                                   cudaStream_t s) {
   if (a.nseg != 1 || a.out_format != 0 || a.bulk_store || a.fp6 || a.s8)
     return cudaErrorInvalidValue;
-  return a.out_fp16 ? launch_herk_t<__half, true>(tmQ, a, grid, s)
-                    : launch_herk_t<float, true>(tmQ, a, grid, s);
+  return a.out_fp16 ? launch_herk_t<__half, true, false>(tmQ, a, grid, s)
+                    : launch_herk_t<float, true, false>(tmQ, a, grid, s);
 }
 
 }  // namespace ftdx

@@ -39,6 +39,12 @@ constexpr int kStgRowBytes = kTile * 8 + 16;
 constexpr int kStgBytes = 2 /*halves*/ * 2 /*buffers*/ * kStgRows * kStgRowBytes;
 constexpr size_t kHerkSmem = 1024 + size_t(kStages) * kStageBytes + kStgBytes + 256;
 static_assert(((kTile / 2) / kStgRows) % 2 == 0, "bulk tiles end on staging buffer 1");
+// Split operands (hi + lo, HerkArgs::nseg = 3): the ring's stages are units, the
+// Re and Im planes of one part of one block; no bulk-store staging.
+constexpr int kUnitBytes = 2 * kPlaneBytes;
+constexpr int kSplitUnits = 7;
+constexpr size_t kSplitSmem = 1024 + size_t(kSplitUnits) * kUnitBytes + 256;
+static_assert(kSplitSmem <= 232448, "shared memory per CTA");
 // Fused promotion (store-mode flag kStoreFused, QC input): the producer loads
 // raw QC bytes by TMA and kConvWarps converter warps write the E4M3 operand
 // planes into shared memory, so no operand planes exist in HBM.  Two operand
@@ -172,6 +178,9 @@ cudaError_t ensure_smem_limit(const void* kernel, size_t bytes);
 // the calling thread; ftdx_last_error(NULL) returns it (ftdx_api.cu).
 void set_thread_error(const char* fmt, ...);
 
+// Rows per block of a promotion pass over `rows` rows of `chunks` per-thread
+// pieces (herk_fp8.cu).
+int promotion_rows_per_block(int64_t rows, int chunks);
 // Host-side launchers (herk_fp8.cu).
 // neg_plane: also write plane 2 = -Re (CTA-pair kernel operand)
 cudaError_t launch_qc_to_planes(const uint8_t* qc, uint8_t* z, int64_t rows, int K, int Kp,
@@ -259,7 +268,7 @@ cudaError_t launch_nvfp4(const void* A, int64_t rows, int K, int n, int batch, u
 // needs that placement; any other takes the three-kernel path).
 cudaError_t launch_float_to_planes(const void* a, uint8_t* z, int64_t rows, int K, int Kp,
                                    int zpitch, int n, int batch, int split, int neg,
-                                   float* qscale, float* out_scale, uint32_t* amax_bits,
+                                   float* out_scale, uint32_t* amax_bits,
                                    uint32_t* arrive, uint32_t* status, int sm_count,
                                    cudaStream_t s);
 
