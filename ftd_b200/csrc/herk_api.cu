@@ -180,7 +180,7 @@ ftdx_status prepare(ftdx_handle h, const HerkCall& c, cudaStream_t s, const Plan
       fused ? FTDX_OK : ensure_workspace(h, size_t((pair ? 3 : 2) * rows * zpitch), s);
   if (st != FTDX_OK) return st;
   if (c.input == FTDX_IN_FP32) {
-    st = ensure_aux(h, size_t(140) * size_t(c.batch) + 256, s);
+    st = ensure_aux(h, size_t(136) * size_t(c.batch) + 256, s);
     if (st != FTDX_OK) return st;
   }
   if (splits > 1) {
@@ -284,11 +284,10 @@ ftdx_status launch_all(ftdx_handle h, const HerkCall& c, const Strategy& strat, 
   const int64_t rows = int64_t(c.N) * c.batch;
   const bool fp6 = ((strat.store_mode & kStoreFp6) || c.compute == FTDX_COMPUTE_FP6) && fp6_ok(c);
   const bool s8 = !fp6 && pair && (strat.store_mode & kStoreS8) && fp6_ok(c);
-  // float inputs: arrival words (32 per channel), amax, qscale, out_scale
+  // float inputs: arrival words (32 per channel), amax, out_scale
   uint32_t* arrive = reinterpret_cast<uint32_t*>(h->aux);
   uint32_t* amax = arrive + int64_t(c.batch) * 32;
-  float* qscale = reinterpret_cast<float*>(amax + c.batch);
-  float* out_scale = qscale + c.batch;
+  float* out_scale = reinterpret_cast<float*>(amax + c.batch);
   cudaError_t e = cudaSuccess;
   if (!fused) {
     ScopedTimer tm(h, s, 1);
@@ -322,7 +321,7 @@ ftdx_status launch_all(ftdx_handle h, const HerkCall& c, const Strategy& strat, 
         if (e == cudaSuccess && pair) e = launch_negate_plane(h->z, rows * zpitch, h->sm_count, s);
       } else {
         e = launch_float_to_planes(c.A, h->z, rows, c.K, int(Kp), int(zpitch), c.N, c.batch,
-                                   is_split(c) ? 1 : 0, pair ? 1 : 0, qscale, out_scale, amax,
+                                   is_split(c) ? 1 : 0, pair ? 1 : 0, out_scale, amax,
                                    arrive, h->d_status, h->sm_count, s);
       }
     }

@@ -265,7 +265,7 @@ cudaError_t launch_nvfp4(const void* A, int64_t rows, int K, int n, int batch, u
 // Float complex [rows][K] -> scaled E4M3 planes of pitch zpitch (precision.cu);
 // neg: also plane 2 (-Re).  arrive: 32 words per channel, 128-byte aligned,
 // directly followed by amax_bits[batch] (the one-pass cooperative kernel
-// needs that placement; any other takes the three-kernel path).
+// needs that placement; any other takes the two-kernel path).
 cudaError_t launch_float_to_planes(const void* a, uint8_t* z, int64_t rows, int K, int Kp,
                                    int zpitch, int n, int batch, int split, int neg,
                                    float* out_scale, uint32_t* amax_bits,

@@ -3,7 +3,7 @@
 //
 //   amax pass   : per channel, the largest |Re| or |Im| (atomicMax on the
 //                 bit patterns of non-negative floats, which order like ints)
-//   scale pass  : s_c = 448 / amax_c (448 = largest finite E4M3); the
+//   scale       : s_c = 448 / amax_c (448 = largest finite E4M3); the
 //                 correlator multiplies channel c's result by 1 / s_c^2
 //   quantise    : hi = E4M3(s_c x) (round to nearest even, saturating) into
 //                 columns [0, Kp) of the planes; in split mode also
@@ -11,13 +11,14 @@
 //                 correlator's K segments (hi,hi) + (hi,lo) + (lo,hi) this
 //                 carries about 7 significant bits per sample instead of 4.
 //
-// In the plain mode the three passes run as one cooperative persistent
-// kernel (scale_quantize_kernel) when the device can hold its grid: each
+// In the plain mode large channels take one cooperative persistent kernel
+// (scale_quantize_kernel) when the device can hold its grid: each
 // block takes the same share of every channel, finds the amax of its share
 // of channel c while it quantises its share of channel c - 1, which it read
 // one channel earlier and which is still in L2, so HBM sees the input once.
-// The split mode, and a grid that cannot be co-resident, use three kernels
-// (amax, scale, quantise) that read it twice.
+// Small channels (launch_float_to_planes says which), the split mode, and a
+// grid that cannot be co-resident, use two kernels (amax, quantise) that read
+// it twice.
 #include <cuda_fp16.h>
 #include <cuda_fp8.h>
 
@@ -72,14 +73,10 @@ __global__ void __launch_bounds__(256) amax_kernel(const float2* __restrict__ a,
   }
 }
 
-__global__ void scale_kernel(const uint32_t* __restrict__ amax_bits, int batch,
-                             float* __restrict__ qscale, float* __restrict__ out_scale) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= batch) return;
-  const float m = __uint_as_float(amax_bits[c]);
-  const float s = (m > 0.f && m < 3.0e38f) ? 448.f / m : 1.f;
-  qscale[c] = s;
-  out_scale[c] = 1.f / (s * s);
+// A channel's scale from its largest component; the correlator multiplies its
+// result by 1 / scale^2.
+__device__ __forceinline__ float channel_scale(float amax) {
+  return (amax > 0.f && amax < 3.0e38f) ? 448.f / amax : 1.f;
 }
 
 __device__ __forceinline__ uint32_t e4m3x2(float a, float b) {
@@ -90,13 +87,15 @@ __device__ __forceinline__ float e4m3_to_float(uint32_t byte) {
   return __half2float(__half(hr));
 }
 
-// One thread quantises 8 samples of one row.  With `vec` (uniform: K even
+// One thread quantises 8 samples of one row; the thread with a channel's first
+// samples stores its out_scale.  With `vec` (uniform: K even
 // and the input 16-byte aligned) a row's 8 samples are read as four 16-byte
 // loads; otherwise, and past K, one sample at a time.
 __global__ void __launch_bounds__(256) quantize_kernel(const float2* __restrict__ a,
                                                        uint8_t* __restrict__ z, int64_t rows,
                                                        int K, int Kp, int zpitch, int n,
-                                                       const float* __restrict__ qscale, int split,
+                                                       const uint32_t* __restrict__ amax_bits,
+                                                       float* __restrict__ out_scale, int split,
                                                        int rows_per_block, int vec) {
   const int chunks = Kp >> 3;
   const int64_t r0 = int64_t(blockIdx.x) * rows_per_block;
@@ -105,11 +104,18 @@ __global__ void __launch_bounds__(256) quantize_kernel(const float2* __restrict_
   const int64_t plane = rows * int64_t(zpitch);
   // the block's rows belong to at most a few channels: 32-bit channel index
   const int c0 = int(r0 / n), rin0 = int(r0 - int64_t(c0) * n);
+  int cs = -1;  // the channel s belongs to
+  float s = 1.f;
   for (int l = threadIdx.x; l < nloc; l += blockDim.x) {
     const int rl = l / chunks;
     const int t0 = (l - rl * chunks) << 3;
     const int64_t r = r0 + rl;
-    const float s = qscale[c0 + (rin0 + rl) / n];
+    const int c = c0 + (rin0 + rl) / n;
+    if (c != cs) {
+      s = channel_scale(__uint_as_float(__ldg(amax_bits + c)));
+      cs = c;
+    }
+    if (t0 == 0 && r == int64_t(c) * n) out_scale[c] = 1.f / (s * s);
     float xr[8], xi[8];
     const float2* src = a + r * K + t0;
     if (vec && t0 + 8 <= K) {
@@ -231,10 +237,9 @@ __device__ __forceinline__ int u1_len(int64_t u0, int64_t per_blk, int64_t units
 // Thread 0 of a block of scale_quantize_kernel: wait until every block has
 // counted its amax of channel cq into its arrival word (acquire; bounded by
 // FTDX_WAIT_NS, after which the status word gets kStatusTimeoutOther and the
-// block's later waits are skipped), then the channel's scale s = 448 / amax
-// as scale_kernel (block 0 also stores qscale and out_scale).
-__device__ __forceinline__ float wait_channel_scale(int cq, float* __restrict__ qscale,
-                                                    float* __restrict__ out_scale,
+// block's later waits are skipped), then the channel's scale (block 0 also
+// stores its out_scale).
+__device__ __forceinline__ float wait_channel_scale(int cq, float* __restrict__ out_scale,
                                                     uint32_t* amax_bits, uint32_t* arrive_word,
                                                     uint32_t* status, bool& aborted) {
   if (!aborted && !dev::flag_wait_limit(arrive_word, gridDim.x, FTDX_WAIT_NS)) {
@@ -244,11 +249,8 @@ __device__ __forceinline__ float wait_channel_scale(int cq, float* __restrict__ 
   uint32_t mb;
   asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(mb) : "l"(amax_bits + cq) : "memory");
   const float mx = __uint_as_float(mb);
-  const float sc = (mx > 0.f && mx < 3.0e38f) ? 448.f / mx : 1.f;
-  if (blockIdx.x == 0) {
-    qscale[cq] = sc;
-    out_scale[cq] = 1.f / (sc * sc);
-  }
+  const float sc = channel_scale(mx);
+  if (blockIdx.x == 0) out_scale[cq] = 1.f / (sc * sc);
   return sc;
 }
 
@@ -291,12 +293,11 @@ __device__ __forceinline__ void quantise_unit(float (&xr)[8], float (&xi)[8], fl
 // no closing barrier.  A unit is re-read about one channel of reads (n K
 // samples) after its first read, so the re-read hits L2 while a channel is
 // well below the L2's size.  neg: also write plane 2 = plane 0 with every
-// sign flipped.  Per-element arithmetic is that of the three-kernel path,
+// sign flipped.  Per-element arithmetic is that of the two-kernel path,
 // so both give the same bits.
 __global__ void __launch_bounds__(256, 4) scale_quantize_kernel(
     const float2* __restrict__ a, uint8_t* __restrict__ z, int K, int Kp, int zpitch, int n,
-    int batch, int neg, float* __restrict__ qscale, float* __restrict__ out_scale,
-    uint32_t* amax_bits, uint32_t* arrive, uint32_t* status, int vec) {
+    int batch, int neg, float* __restrict__ out_scale, uint32_t* amax_bits, uint32_t* arrive, uint32_t* status, int vec) {
   const int chunks = Kp >> 3;
   const int64_t units = int64_t(n) * chunks;
   const int64_t per_blk = (units + gridDim.x - 1) / gridDim.x;
@@ -347,7 +348,7 @@ __global__ void __launch_bounds__(256, 4) scale_quantize_kernel(
     }
     if (quant_step) {
       if (t == 0)  // 2
-        s_scale[par] = wait_channel_scale(c - 1, qscale, out_scale, amax_bits,
+        s_scale[par] = wait_channel_scale(c - 1, out_scale, amax_bits,
                                           arrive + int64_t(c - 1) * 32, status, aborted);
       __syncthreads();
       sc = s_scale[par];
@@ -425,7 +426,7 @@ cudaError_t launch_channel_amax(const void* a, int64_t per_chan, int batch, uint
 
 cudaError_t launch_float_to_planes(const void* a, uint8_t* z, int64_t rows, int K, int Kp,
                                    int zpitch, int n, int batch, int split, int neg,
-                                   float* qscale, float* out_scale, uint32_t* amax_bits,
+                                   float* out_scale, uint32_t* amax_bits,
                                    uint32_t* arrive, uint32_t* status, int sm_count,
                                    cudaStream_t s) {
   // the arrival words (32 per channel) directly followed by amax_bits: one
@@ -436,9 +437,15 @@ cudaError_t launch_float_to_planes(const void* a, uint8_t* z, int64_t rows, int 
   if (e != cudaSuccess) return e;
   const int vec = (K % 2 == 0) && (reinterpret_cast<uintptr_t>(a) & 15) == 0;
   const int64_t units = int64_t(n) * (Kp >> 3);
-  // the split mode (hi and lo columns) measured faster on the three-kernel
-  // path: 0.91 against 1.02 ms at 4096 x 64 x 1024
-  const int per_sm = split ? 0 : scale_quantize_blocks_per_sm();
+  // The cooperative kernel takes a step per channel, each with a wait for the
+  // whole grid, and saves the second read from HBM: it needs a channel that is
+  // long against the wait, or a single one.  Promotion in us, cooperative / two
+  // kernels: 16 channels of 33.6 MB 205 / 231, 4 of them 64 / 72; 8 of 16.8 MB
+  // 76 / 71; 16 of 8.4 MB 70 / 64, of 4.2 MB 54 / 30, of 1.2 MB 47 / 19; one of
+  // 33.6 MB 20 / 22, of 5.6 MB 12 / 14.  The split mode (hi and lo columns) was
+  // slower on it at any size: 1.02 against 0.91 ms at 4096 x 64 x 1024.
+  const bool large = batch == 1 || int64_t(n) * K * int64_t(sizeof(float2)) >= 24000000;
+  const int per_sm = split || !large ? 0 : scale_quantize_blocks_per_sm();
   if (per_sm > 0 && adjacent && (reinterpret_cast<uintptr_t>(arrive) & 127) == 0 &&
       units < (int64_t(1) << 30)) {
     // at least 256 units (one per thread) per block, at most every resident block
@@ -456,20 +463,19 @@ cudaError_t launch_float_to_planes(const void* a, uint8_t* z, int64_t rows, int 
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     e = cudaLaunchKernelEx(&cfg, scale_quantize_kernel, static_cast<const float2*>(a), z, K, Kp,
-                           zpitch, n, batch, neg, qscale, out_scale, amax_bits, arrive, status,
+                           zpitch, n, batch, neg, out_scale, amax_bits, arrive, status,
                            vec);
     if (e == cudaSuccess) return e;
-    cudaGetLastError();  // not launchable as one cooperative grid: the three-kernel path
+    cudaGetLastError();  // not launchable as one cooperative grid: the two-kernel path
   }
   const int64_t per_chan = int64_t(n) * K;
   e = launch_channel_amax(a, per_chan, batch, amax_bits, sm_count, s);
   if (e != cudaSuccess) return e;
-  scale_kernel<<<(batch + 127) / 128, 128, 0, s>>>(amax_bits, batch, qscale, out_scale);
-  int rpb = 8192 / (Kp >> 3);
-  if (rpb < 1) rpb = 1;
+  const int rpb = promotion_rows_per_block(rows, Kp >> 3);
   const int64_t blocks = (rows + rpb - 1) / rpb;
   quantize_kernel<<<unsigned(blocks), 256, 0, s>>>(static_cast<const float2*>(a), z, rows, K, Kp,
-                                                    zpitch, n, qscale, split, rpb, vec);
+                                                    zpitch, n, amax_bits, out_scale, split, rpb,
+                                                    vec);
   e = cudaGetLastError();
   if (e == cudaSuccess && neg) e = launch_negate_plane(z, rows * zpitch, sm_count, s);
   return e;
