@@ -94,6 +94,7 @@ __global__ void __launch_bounds__(256) adjoint_prepare_kernel(
     const float2* __restrict__ G, __nv_bfloat16* __restrict__ S, int n, int64_t plane_elems,
     int pairs, const uint8_t* __restrict__ V, __nv_bfloat16* __restrict__ VP, int K, int Kp,
     int64_t v_plane) {
+  griddep_launch();
   __shared__ float2 tile[2][32][33];  // [0] = G tile (i, j), [1] = G tile (j, i)
   const int b = blockIdx.y;
   const int r = blockIdx.x;  // lower-triangle tile index -> (ti, tj), tj <= ti
@@ -228,6 +229,7 @@ __global__ void __launch_bounds__(kAThreads, 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  griddep_wait();  // S and V
   const int per_chan = args.tiles_t * args.tiles_a;
   const int kblocks = (args.n + kAK - 1) / kAK;
 
@@ -470,8 +472,8 @@ cudaError_t launch_adjoint(const void* G, const uint8_t* V, void* dV, int n, int
   e = ensure_smem_limit(reinterpret_cast<const void*>(adjoint_tc_kernel), kASmem);
   if (e != cudaSuccess) return e;
   const int grid = a.num_tiles < sm_count ? a.num_tiles : sm_count;
-  adjoint_tc_kernel<<<grid, kAThreads, kASmem, s>>>(tmV, tmS, tmT, a);
-  return cudaGetLastError();
+  return launch_after(a.num_tiles <= 4 * sm_count, adjoint_tc_kernel, dim3(unsigned(grid)), dim3(kAThreads), kASmem, s, tmV, tmS,
+                      tmT, a);
 }
 
 }  // namespace ftdx

@@ -178,6 +178,8 @@ ftdx_status launch_v(ftdx_handle h, const VCall& c, const Strategy& strat, cudaS
   args.alpha = c.alpha;
   args.beta = c.beta;
   args.status = h->d_status;
+  const bool early =
+      int64_t(args.num_tiles) * (p->kp / kStageK) <= kEarlyKBlocks * int64_t(h->sm_count);
   if (pair) {
     // persistent pairs, at most as many as can be resident together
     const int limit = pair_grid_limit(h);
@@ -185,13 +187,13 @@ ftdx_status launch_v(ftdx_handle h, const VCall& c, const Strategy& strat, cudaS
     if (strat.grid < 0) grid = 2 * p->num_tiles_pair;
     grid = std::min(grid, 2 * p->num_tiles_pair) & ~1;
     ScopedTimer tm(h, s, 0);
-    e = launch_herk_fp8_pair(tmZ, args, grid, s);
+    e = launch_herk_fp8_pair(tmZ, args, grid, s, early);
   } else {
     int grid = strat.grid > 0 ? std::min(strat.grid, h->sm_count) : h->sm_count;
     if (strat.grid < 0) grid = p->num_tiles;
     grid = std::min(grid, p->num_tiles);
     ScopedTimer tm(h, s, 0);
-    e = launch_herk_fp8(tmZ, args, grid, s);
+    e = launch_herk_fp8(tmZ, args, grid, s, early);
   }
   if (e != cudaSuccess) return cuda_fail(h, e, "correlator kernel launch");
   return FTDX_OK;

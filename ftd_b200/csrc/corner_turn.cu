@@ -17,6 +17,7 @@
 
 #include "herk_fp8.cuh"
 #include "qc_codec.cuh"
+#include "sm100.cuh"
 
 namespace ftdx {
 namespace {
@@ -51,6 +52,7 @@ __device__ __forceinline__ void put32(uint8_t* dst, const uint32_t (&w)[8], int 
 __global__ void __launch_bounds__(256, 8) ftd_tacp_to_planes_kernel(const uint8_t* __restrict__ raw,
                                                                  uint8_t* __restrict__ z,
                                                                  FtdGeom g) {
+  dev::griddep_launch();
   __shared__ __align__(16) uint8_t tileT[kTS * kTPitch];
   const int64_t S = int64_t(g.n_ant) * g.n_chan * g.n_pol;
   const int64_t s0 = int64_t(blockIdx.x) * kTS;
@@ -149,6 +151,7 @@ __global__ void __launch_bounds__(256, 8) ftd_tacp_to_planes_kernel(const uint8_
 __global__ void __launch_bounds__(256) ftd_cpat_to_planes_kernel(const uint8_t* __restrict__ raw,
                                                                  uint8_t* __restrict__ z,
                                                                  FtdGeom g) {
+  dev::griddep_launch();
   const int chunks = g.Kp >> 4;
   const int64_t total = g.rows * chunks;
   const int n_seg = g.pol_sum ? g.n_pol : 1;

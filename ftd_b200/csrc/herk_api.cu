@@ -362,6 +362,8 @@ ftdx_status launch_all(ftdx_handle h, const HerkCall& c, const Strategy& strat, 
     args.beta = 0.f;
     args.chan_scale = nullptr;
   }
+  const bool early = int64_t(plan->num_tiles) * (Kp / kStageK) * args.nseg <=
+                     kEarlyKBlocks * splits * h->sm_count;
   if (pair) {
     // persistent pairs, at most as many as can be resident together
     const int limit = pair_grid_limit(h);
@@ -369,14 +371,15 @@ ftdx_status launch_all(ftdx_handle h, const HerkCall& c, const Strategy& strat, 
     if (strat.grid < 0) grid = 2 * plan->num_tiles;
     grid = std::min(grid, 2 * plan->num_tiles) & ~1;
     ScopedTimer tm(h, s, 0);
-    e = launch_herk_fp8_pair(tmZ, args, grid, s);
+    e = launch_herk_fp8_pair(tmZ, args, grid, s, early);
   } else {
     int grid = strat.grid > 0 ? strat.grid : h->sm_count;
     if (grid > h->sm_count) grid = h->sm_count;  // persistent: at most one CTA per SM
     if (strat.grid < 0) grid = plan->num_tiles;   // one tile per CTA
     if (grid > plan->num_tiles) grid = plan->num_tiles;
     ScopedTimer tm(h, s, 0);
-    e = fused ? launch_herk_fp8_fused(tmZ, args, grid, s) : launch_herk_fp8(tmZ, args, grid, s);
+    e = fused ? launch_herk_fp8_fused(tmZ, args, grid, s, early)
+              : launch_herk_fp8(tmZ, args, grid, s, early);
   }
   if (e != cudaSuccess) return cuda_fail(h, e, "correlator kernel launch");
   if (splits > 1) {

@@ -235,6 +235,7 @@ constexpr double kRfiThreshold = 25.0;
 __global__ void __launch_bounds__(256) nvfp4_stats_kernel(
     const float2* __restrict__ a, float* __restrict__ power, float* __restrict__ rscale,
     uint32_t* __restrict__ flags, int64_t rows, int K, int n, int fwords, int rfi) {
+  griddep_launch();
   const int lane = threadIdx.x & 31;
   // rows of an even K at a 16-byte aligned base: two samples per load
   const bool vec = (K & 1) == 0 && (reinterpret_cast<uintptr_t>(a) & 15) == 0;
@@ -317,6 +318,8 @@ __global__ void __launch_bounds__(1024) nvfp4_order_kernel(const uint32_t* __res
                                                            int32_t* __restrict__ nflag,
                                                            ChanDesc* __restrict__ chans, int K,
                                                            int kp, int fwords, int split) {
+  griddep_wait();  // the flags
+  griddep_launch();
   __shared__ int s_cnt[32];
   __shared__ int s_total;
   const int c = blockIdx.x;
@@ -384,6 +387,8 @@ __global__ void __launch_bounds__(256, kStaged ? 3 : 4) nvfp4_quant_kernel(
     const int32_t* __restrict__ nflag, const ChanDesc* __restrict__ chans,
     const float* __restrict__ rscale, uint8_t* __restrict__ z, uint8_t* __restrict__ sfa,
     uint8_t* __restrict__ sfb, int64_t rows, int K, int kp, int pitch, SfGeom sg) {
+  griddep_wait();  // row scales and time order
+  griddep_launch();
   const int lane = threadIdx.x & 31;
   extern __shared__ __align__(16) uint8_t stage_smem[];  // kStaged: a row per warp
   const int blocks_per_row = pitch / 8;  // 8 bytes of E2M1 per block
@@ -702,6 +707,7 @@ __global__ void __launch_bounds__(k4Threads, 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  griddep_wait();  // operands, scales and the channels' lo extents
 
   if (warp == 0) {
     // ------------------------------------------------ TMA producer
@@ -900,6 +906,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(k4pThreads, 1)
   cluster_sync_all();  // both CTAs' barriers exist before any cross-CTA signal
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  griddep_wait();  // operands, scales and the channels' lo extents
 
   if (warp == 0) {
     // ------------------------------------------------ TMA producer (both CTAs)
@@ -1103,6 +1110,8 @@ cudaError_t launch_nvfp4(const void* A, int64_t rows, int K, int n, int batch, u
   auto encode = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(encode_fn);
   if (!encode) return cudaErrorInvalidValue;
   if (pair && nvfp4_pair_limit() < 1) return cudaErrorInvalidConfiguration;
+  const bool early =
+      int64_t(num_tiles) * nvfp4_kblocks(K) <= kEarlyKBlocks * int64_t(sm_count);
   const Fp4Ws w = fp4_ws(n, batch, K, pair);
   const int64_t pitch = w.pitch, rpitch = w.rpitch;  // one half (hi or lo), whole row
   uint8_t* z = ws;
@@ -1128,24 +1137,23 @@ cudaError_t launch_nvfp4(const void* A, int64_t rows, int K, int n, int batch, u
     nvfp4_stats_kernel<<<unsigned(blocks), 256, 0, s>>>(static_cast<const float2*>(A), power,
                                                         rscale, flags, rows, K, n, w.fwords, rfi);
     // time order and lo extent of every channel (written into the plan's table)
-    nvfp4_order_kernel<<<unsigned(batch), 1024, 0, s>>>(flags, src, nflag,
-                                                        const_cast<ChanDesc*>(chans), K,
-                                                        int(w.kp), w.fwords, split);
+    e = launch_after(early, nvfp4_order_kernel, dim3(unsigned(batch)), dim3(1024), 0, s, flags, src, nflag,
+                     const_cast<ChanDesc*>(chans), K, int(w.kp), w.fwords, split);
+    if (e != cudaSuccess) return e;
     // E2M1 operands and UE4M3 scale atoms
     auto quantise = [&](auto kernel, size_t smem) {
-      kernel<<<unsigned(blocks), 256, smem, s>>>(static_cast<const float2*>(A), src, nflag, chans,
-                                                 rscale, z, sfa, sfb, rows, K, int(w.kp),
-                                                 int(pitch), w.sg);
+      return launch_after(early, kernel, dim3(unsigned(blocks)), dim3(256), smem, s,
+                          static_cast<const float2*>(A), src, nflag, chans, rscale, z, sfa, sfb,
+                          rows, K, int(w.kp), int(pitch), w.sg);
     };
     if (K <= kStageSamples) {
       e = ensure_smem_limit(reinterpret_cast<const void*>(nvfp4_quant_kernel<true>),
                             8 * stage_bytes_per_row(kStageSamples));
       if (e != cudaSuccess) return e;
-      quantise(nvfp4_quant_kernel<true>, 8 * stage_bytes_per_row(K));
+      e = quantise(nvfp4_quant_kernel<true>, 8 * stage_bytes_per_row(K));
     } else {
-      quantise(nvfp4_quant_kernel<false>, 0);
+      e = quantise(nvfp4_quant_kernel<false>, 0);
     }
-    e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }
   if (!(phases & 2)) return cudaSuccess;
@@ -1177,14 +1185,14 @@ cudaError_t launch_nvfp4(const void* A, int64_t rows, int K, int n, int batch, u
   if (pair) {
     const int limit = nvfp4_pair_limit();
     const int pairs = num_tiles < limit ? num_tiles : limit;
-    herk_fp4_pair_kernel<<<2 * pairs, k4pThreads, k4pSmem, s>>>(tmA, tmB, tmSa, tmSb, args);
-    return cudaGetLastError();
+    return launch_after(early, herk_fp4_pair_kernel, dim3(unsigned(2 * pairs)), dim3(k4pThreads), k4pSmem, s,
+                        tmA, tmB, tmSa, tmSb, args);
   }
   e = ensure_smem_limit(reinterpret_cast<const void*>(herk_fp4_tc_kernel), k4Smem);
   if (e != cudaSuccess) return e;
   const int grid = num_tiles < sm_count ? num_tiles : sm_count;
-  herk_fp4_tc_kernel<<<grid, k4Threads, k4Smem, s>>>(tmA, tmB, args);
-  return cudaGetLastError();
+  return launch_after(early, herk_fp4_tc_kernel, dim3(unsigned(grid)), dim3(k4Threads), k4Smem, s, tmA, tmB,
+                      args);
 }
 
 }  // namespace ftdx

@@ -37,6 +37,7 @@ __global__ void __launch_bounds__(256) qc_to_planes_kernel(const uint8_t* __rest
                                                            uint8_t* __restrict__ z, int64_t rows,
                                                            int K, int Kp, int rows_per_block,
                                                            int neg_plane) {
+  griddep_launch();
   const int chunks = Kp >> 4;
   const int64_t r0 = int64_t(blockIdx.x) * rows_per_block;
   const int64_t nrows64 = rows - r0 < rows_per_block ? rows - r0 : rows_per_block;
@@ -69,6 +70,7 @@ __global__ void __launch_bounds__(256) qc_to_planes_s8_kernel(const uint8_t* __r
                                                               uint8_t* __restrict__ z,
                                                               int64_t rows, int K, int Kp,
                                                               int rows_per_block, int neg_plane) {
+  griddep_launch();
   const int chunks = Kp >> 4;
   const int64_t r0 = int64_t(blockIdx.x) * rows_per_block;
   const int64_t nrows64 = rows - r0 < rows_per_block ? rows - r0 : rows_per_block;
@@ -100,6 +102,7 @@ __global__ void __launch_bounds__(256) qc_to_planes6_kernel(const uint8_t* __res
                                                             uint8_t* __restrict__ z, int64_t rows,
                                                             int K, int Kp, int rows_per_block,
                                                             int neg_plane) {
+  griddep_launch();
   const int chunks = Kp >> 4;
   const int64_t pitch = int64_t(Kp) * 3 / 4;
   const int64_t r0 = int64_t(blockIdx.x) * rows_per_block;
@@ -136,6 +139,8 @@ __global__ void __launch_bounds__(256) qc_to_planes6_kernel(const uint8_t* __res
 // Plane 2 = plane 0 with every E4M3 sign flipped (-Re), for inputs whose
 // promotion kernel writes two planes.  n16 = plane bytes / 16.
 __global__ void __launch_bounds__(256) negate_plane_kernel(uint4* __restrict__ z, int64_t n16) {
+  griddep_wait();  // reads what the promotion before it wrote
+  griddep_launch();
   constexpr uint32_t kS = 0x80808080u;
   for (int64_t x = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; x < n16;
        x += int64_t(gridDim.x) * blockDim.x) {
@@ -159,6 +164,7 @@ __global__ void __launch_bounds__(256) fp16_to_planes_kernel(const __half2* __re
                                                              uint8_t* __restrict__ z, int64_t rows,
                                                              int K, int Kp, int rows_per_block,
                                                              int vec) {
+  griddep_launch();
   const int chunks = Kp >> 3;  // 8 samples per thread
   const int64_t r0 = int64_t(blockIdx.x) * rows_per_block;
   const int64_t nrows64 = rows - r0 < rows_per_block ? rows - r0 : rows_per_block;
@@ -207,6 +213,7 @@ __global__ void __launch_bounds__(256) gather_qc_to_planes_kernel(const GatherDe
                                                                   int64_t total_rows, int Kp,
                                                                   int rows_per_block,
                                                                   int neg_plane) {
+  griddep_launch();
   const GatherDesc g = gd[blockIdx.y];
   const int r0 = blockIdx.x * rows_per_block;
   if (r0 >= g.n) return;
@@ -410,6 +417,8 @@ __global__ void __launch_bounds__(kFused ? kFusedThreads : kHerkThreads, 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  griddep_wait();    // the operand planes (or nothing: the caller's input)
+  griddep_launch();  // the split-K reduction
 
   if (warp == 0) {
     // ------------------------------------------------ TMA producer
@@ -947,6 +956,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kHerkThreads, 1)
   cluster_sync_all();  // both CTAs' barriers exist before any cross-CTA signal
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  griddep_wait();    // the operand planes
+  griddep_launch();  // the split-K reduction
 
   if (warp == 0) {
     // ------------------------------------------------ TMA producer (both CTAs)
@@ -1270,8 +1281,8 @@ cudaError_t launch_negate_plane(uint8_t* z, int64_t plane_bytes, int sm_count, c
   int64_t blocks = (n16 + 255) / 256;
   if (blocks > int64_t(sm_count) * 8) blocks = int64_t(sm_count) * 8;
   if (blocks < 1) blocks = 1;
-  negate_plane_kernel<<<unsigned(blocks), 256, 0, s>>>(reinterpret_cast<uint4*>(z), n16);
-  return cudaGetLastError();
+  return launch_after(true, negate_plane_kernel, dim3(unsigned(blocks)), dim3(256), 0, s,
+                      reinterpret_cast<uint4*>(z), n16);
 }
 
 cudaError_t launch_fp16_to_planes(const void* a16, uint8_t* z, int64_t rows, int K, int Kp,
@@ -1294,14 +1305,14 @@ cudaError_t launch_gather_qc_to_planes(const GatherDesc* g, int nch, int max_n, 
 
 template <typename OutT, bool kFused, bool kSplit>
 static cudaError_t launch_herk_t(const CUtensorMap& tmZ, const HerkArgs& a, int grid,
-                                 cudaStream_t s) {
+                                 cudaStream_t s, bool early) {
   constexpr size_t smem = kFused ? kFusedSmem : (kSplit ? kSplitSmem : kHerkSmem);
   constexpr int threads = kFused ? kFusedThreads : kHerkThreads;
   cudaError_t e = ensure_smem_limit(
       reinterpret_cast<const void*>(herk_fp8_tc_kernel<OutT, kFused, kSplit>), smem);
   if (e != cudaSuccess) return e;
-  herk_fp8_tc_kernel<OutT, kFused, kSplit><<<grid, threads, smem, s>>>(tmZ, a);
-  return cudaGetLastError();
+  return launch_after(early, herk_fp8_tc_kernel<OutT, kFused, kSplit>, dim3(unsigned(grid)),
+                      dim3(threads), smem, s, tmZ, a);
 }
 
 template <typename OutT>
@@ -1311,11 +1322,11 @@ static cudaError_t pair_attributes() {
 
 template <typename OutT>
 static cudaError_t launch_pair_t(const CUtensorMap& tmZ, const HerkArgs& a, int grid,
-                                 cudaStream_t s) {
+                                 cudaStream_t s, bool early) {
   cudaError_t e = pair_attributes<OutT>();
   if (e != cudaSuccess) return e;
-  herk_fp8_pair_kernel<OutT><<<grid, kHerkThreads, kPairSmem, s>>>(tmZ, a);
-  return cudaGetLastError();
+  return launch_after(early, herk_fp8_pair_kernel<OutT>, dim3(unsigned(grid)), dim3(kHerkThreads),
+                      kPairSmem, s, tmZ, a);
 }
 
 cudaError_t herk_fp8_pair_max_clusters(int sm_count, int* clusters) {
@@ -1334,9 +1345,10 @@ cudaError_t herk_fp8_pair_max_clusters(int sm_count, int* clusters) {
 }
 
 cudaError_t launch_herk_fp8_pair(const CUtensorMap& tmZ, const HerkArgs& a, int grid,
-                                 cudaStream_t s) {
+                                 cudaStream_t s, bool early) {
   if (grid < 2 || (grid & 1)) return cudaErrorInvalidConfiguration;
-  return a.out_fp16 ? launch_pair_t<__half>(tmZ, a, grid, s) : launch_pair_t<float>(tmZ, a, grid, s);
+  return a.out_fp16 ? launch_pair_t<__half>(tmZ, a, grid, s, early)
+                    : launch_pair_t<float>(tmZ, a, grid, s, early);
 }
 
 // Split-K: the correlator wrote `splits` partial triangles per channel
@@ -1348,6 +1360,7 @@ __global__ void __launch_bounds__(256) split_reduce_kernel(const float2* __restr
                                                            int batch, int splits, float alpha,
                                                            float beta,
                                                            const float* __restrict__ chan_scale) {
+  griddep_wait();
   const int64_t total = int64_t(batch) * P;
   for (int64_t x = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; x < total;
        x += int64_t(gridDim.x) * blockDim.x) {
@@ -1386,31 +1399,32 @@ cudaError_t launch_split_reduce(const float2* ws, void* out, int out_fp16, int64
   int64_t blocks = (total + 255) / 256;
   if (blocks > int64_t(sm_count) * 16) blocks = int64_t(sm_count) * 16;
   if (blocks < 1) blocks = 1;
-  if (out_fp16)
-    split_reduce_kernel<__half2><<<unsigned(blocks), 256, 0, s>>>(
-        ws, static_cast<__half2*>(out), P, batch, splits, alpha, beta, chan_scale);
-  else
-    split_reduce_kernel<float2><<<unsigned(blocks), 256, 0, s>>>(
-        ws, static_cast<float2*>(out), P, batch, splits, alpha, beta, chan_scale);
-  return cudaGetLastError();
+  const dim3 grid{unsigned(blocks)}, block{256};
+  return out_fp16 ? launch_after(true, split_reduce_kernel<__half2>, grid, block, 0, s, ws,
+                                 static_cast<__half2*>(out), P, batch, splits, alpha, beta,
+                                 chan_scale)
+                  : launch_after(true, split_reduce_kernel<float2>, grid, block, 0, s, ws,
+                                 static_cast<float2*>(out), P, batch, splits, alpha, beta,
+                                 chan_scale);
 }
 
-cudaError_t launch_herk_fp8(const CUtensorMap& tmZ, const HerkArgs& a, int grid, cudaStream_t s) {
+cudaError_t launch_herk_fp8(const CUtensorMap& tmZ, const HerkArgs& a, int grid, cudaStream_t s,
+                            bool early) {
   if (a.nseg != 1) {  // (hi, hi), (hi, lo), (lo, hi)
     if (a.nseg != 3 || a.out_format != 0 || a.fp6) return cudaErrorInvalidValue;
-    return a.out_fp16 ? launch_herk_t<__half, false, true>(tmZ, a, grid, s)
-                      : launch_herk_t<float, false, true>(tmZ, a, grid, s);
+    return a.out_fp16 ? launch_herk_t<__half, false, true>(tmZ, a, grid, s, early)
+                      : launch_herk_t<float, false, true>(tmZ, a, grid, s, early);
   }
-  return a.out_fp16 ? launch_herk_t<__half, false, false>(tmZ, a, grid, s)
-                    : launch_herk_t<float, false, false>(tmZ, a, grid, s);
+  return a.out_fp16 ? launch_herk_t<__half, false, false>(tmZ, a, grid, s, early)
+                    : launch_herk_t<float, false, false>(tmZ, a, grid, s, early);
 }
 
 cudaError_t launch_herk_fp8_fused(const CUtensorMap& tmQ, const HerkArgs& a, int grid,
-                                  cudaStream_t s) {
+                                  cudaStream_t s, bool early) {
   if (a.nseg != 1 || a.out_format != 0 || a.bulk_store || a.fp6 || a.s8)
     return cudaErrorInvalidValue;
-  return a.out_fp16 ? launch_herk_t<__half, true, false>(tmQ, a, grid, s)
-                    : launch_herk_t<float, true, false>(tmQ, a, grid, s);
+  return a.out_fp16 ? launch_herk_t<__half, true, false>(tmQ, a, grid, s, early)
+                    : launch_herk_t<float, true, false>(tmQ, a, grid, s, early);
 }
 
 }  // namespace ftdx

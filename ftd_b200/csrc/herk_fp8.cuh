@@ -181,6 +181,31 @@ void set_thread_error(const char* fmt, ...);
 // Rows per block of a promotion pass over `rows` rows of `chunks` per-thread
 // pieces (herk_fp8.cu).
 int promotion_rows_per_block(int64_t rows, int chunks);
+// Launches `kernel`, which calls griddep_wait() before it touches anything that
+// the kernel queued before it writes: its start (barriers, TMEM, descriptor
+// prefetch) then overlaps that kernel's end.  Without such a kernel in front, or
+// with early = false, it starts as any launch does.
+// The gap between two dependent launches is 2 to 4 us: 24 channels of 702 x 500
+// to FP16 take 30.6 us without and 26.7 with an early start, 16 of 1024 x 1024
+// FP16 samples 59.4 and 58.1.  Kernels of 200 us and more lose 0.5 to 1% by it
+// (their blocks take their SMs in the order in which the kernel before leaves
+// them), so callers ask for it up to kEarlyKBlocks k-blocks per SM.
+constexpr int64_t kEarlyKBlocks = 64;
+template <typename... KArgs, typename... Args>
+cudaError_t launch_after(bool early, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
+                         cudaStream_t s, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = early ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
+}
 // Host-side launchers (herk_fp8.cu).
 // neg_plane: also write plane 2 = -Re (CTA-pair kernel operand)
 cudaError_t launch_qc_to_planes(const uint8_t* qc, uint8_t* z, int64_t rows, int K, int Kp,
@@ -219,12 +244,14 @@ cudaError_t launch_fp16_to_planes(const void* a16, uint8_t* z, int64_t rows, int
 cudaError_t launch_gather_qc_to_planes(const GatherDesc* g, int nch, int max_n, uint8_t* z,
                                        int64_t total_rows, int Kp, cudaStream_t s,
                                        int neg_plane = 0);
-cudaError_t launch_herk_fp8(const CUtensorMap& tmZ, const HerkArgs& a, int grid, cudaStream_t s);
+// early: start while the promotion ends (launch_after).
+cudaError_t launch_herk_fp8(const CUtensorMap& tmZ, const HerkArgs& a, int grid, cudaStream_t s,
+                            bool early);
 // The single-CTA kernel with fused promotion: tmQ maps the raw QC bytes
 // [rows][K] (2-D, 128 x 128-byte boxes, no swizzle); a.nseg must be 1,
 // a.out_format 0 and a.bulk_store 0.
 cudaError_t launch_herk_fp8_fused(const CUtensorMap& tmQ, const HerkArgs& a, int grid,
-                                  cudaStream_t s);
+                                  cudaStream_t s, bool early);
 // Split-K reduction: C[c] = alpha * cs_c * sum_s ws[c*splits + s] + beta * C[c].
 cudaError_t launch_split_reduce(const float2* ws, void* out, int out_fp16, int64_t P, int batch,
                                 int splits, float alpha, float beta, const float* chan_scale,
@@ -233,7 +260,7 @@ cudaError_t launch_split_reduce(const float2* ws, void* out, int out_fp16, int64
 // 256-input blocks); tmZ covers three planes (Re, Im, -Re), boxes of 128
 // rows; grid even.
 cudaError_t launch_herk_fp8_pair(const CUtensorMap& tmZ, const HerkArgs& a, int grid,
-                                 cudaStream_t s);
+                                 cudaStream_t s, bool early);
 // Number of 2-CTA clusters of the pair kernel that fit on the device at once.
 cudaError_t herk_fp8_pair_max_clusters(int sm_count, int* clusters);
 // Gain-calibration loss and gradient over packed triangles (gain_grad.cu).

@@ -196,7 +196,7 @@ extern "C" ftdx_status ftdx_herk_static(const void* A, void* C, int N, int K, in
   args.beta = 0.f;
   args.status = status;
   const int grid = int(std::min<int64_t>(ntiles, sms));
-  e = launch_herk_fp8(tm, args, grid, s);
+  e = launch_herk_fp8(tm, args, grid, s, true);  // small by its scratch
   if (e != cudaSuccess) {
     set_thread_error("ftdx_herk_static: correlator launch failed: %s", cudaGetErrorString(e));
     return FTDX_ERR_CUDA;

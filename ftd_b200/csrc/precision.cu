@@ -35,6 +35,7 @@ namespace {
 // says the channel starts 16-byte aligned and per_chan is even.
 __global__ void __launch_bounds__(256) amax_kernel(const float2* __restrict__ a, int64_t per_chan,
                                                    uint32_t* __restrict__ amax_bits, int vec) {
+  dev::griddep_launch();
   const int c = blockIdx.y;
   const float2* p = a + int64_t(c) * per_chan;
   float m = 0.f;
@@ -97,6 +98,8 @@ __global__ void __launch_bounds__(256) quantize_kernel(const float2* __restrict_
                                                        const uint32_t* __restrict__ amax_bits,
                                                        float* __restrict__ out_scale, int split,
                                                        int rows_per_block, int vec) {
+  dev::griddep_wait();  // the channels' amax
+  dev::griddep_launch();
   const int chunks = Kp >> 3;
   const int64_t r0 = int64_t(blockIdx.x) * rows_per_block;
   const int64_t nrows64 = rows - r0 < rows_per_block ? rows - r0 : rows_per_block;
@@ -298,6 +301,7 @@ __device__ __forceinline__ void quantise_unit(float (&xr)[8], float (&xi)[8], fl
 __global__ void __launch_bounds__(256, 4) scale_quantize_kernel(
     const float2* __restrict__ a, uint8_t* __restrict__ z, int K, int Kp, int zpitch, int n,
     int batch, int neg, float* __restrict__ out_scale, uint32_t* amax_bits, uint32_t* arrive, uint32_t* status, int vec) {
+  dev::griddep_launch();
   const int chunks = Kp >> 3;
   const int64_t units = int64_t(n) * chunks;
   const int64_t per_blk = (units + gridDim.x - 1) / gridDim.x;
@@ -473,10 +477,9 @@ cudaError_t launch_float_to_planes(const void* a, uint8_t* z, int64_t rows, int 
   if (e != cudaSuccess) return e;
   const int rpb = promotion_rows_per_block(rows, Kp >> 3);
   const int64_t blocks = (rows + rpb - 1) / rpb;
-  quantize_kernel<<<unsigned(blocks), 256, 0, s>>>(static_cast<const float2*>(a), z, rows, K, Kp,
-                                                    zpitch, n, amax_bits, out_scale, split, rpb,
-                                                    vec);
-  e = cudaGetLastError();
+  e = launch_after(rows * K <= (int64_t(8) << 20), quantize_kernel, dim3(unsigned(blocks)), dim3(256), 0, s,
+                   static_cast<const float2*>(a), z, rows, K, Kp, zpitch, n, amax_bits, out_scale,
+                   split, rpb, vec);
   if (e == cudaSuccess && neg) e = launch_negate_plane(z, rows * zpitch, sm_count, s);
   return e;
 }
