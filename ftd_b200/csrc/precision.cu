@@ -88,89 +88,8 @@ __device__ __forceinline__ float e4m3_to_float(uint32_t byte) {
   return __half2float(__half(hr));
 }
 
-// One thread quantises 8 samples of one row; the thread with a channel's first
-// samples stores its out_scale.  With `vec` (uniform: K even
-// and the input 16-byte aligned) a row's 8 samples are read as four 16-byte
-// loads; otherwise, and past K, one sample at a time.
-__global__ void __launch_bounds__(256) quantize_kernel(const float2* __restrict__ a,
-                                                       uint8_t* __restrict__ z, int64_t rows,
-                                                       int K, int Kp, int zpitch, int n,
-                                                       const uint32_t* __restrict__ amax_bits,
-                                                       float* __restrict__ out_scale, int split,
-                                                       int rows_per_block, int vec) {
-  dev::griddep_wait();  // the channels' amax
-  dev::griddep_launch();
-  const int chunks = Kp >> 3;
-  const int64_t r0 = int64_t(blockIdx.x) * rows_per_block;
-  const int64_t nrows64 = rows - r0 < rows_per_block ? rows - r0 : rows_per_block;
-  const int nloc = int(nrows64) * chunks;
-  const int64_t plane = rows * int64_t(zpitch);
-  // the block's rows belong to at most a few channels: 32-bit channel index
-  const int c0 = int(r0 / n), rin0 = int(r0 - int64_t(c0) * n);
-  int cs = -1;  // the channel s belongs to
-  float s = 1.f;
-  for (int l = threadIdx.x; l < nloc; l += blockDim.x) {
-    const int rl = l / chunks;
-    const int t0 = (l - rl * chunks) << 3;
-    const int64_t r = r0 + rl;
-    const int c = c0 + (rin0 + rl) / n;
-    if (c != cs) {
-      s = channel_scale(__uint_as_float(__ldg(amax_bits + c)));
-      cs = c;
-    }
-    if (t0 == 0 && r == int64_t(c) * n) out_scale[c] = 1.f / (s * s);
-    float xr[8], xi[8];
-    const float2* src = a + r * K + t0;
-    if (vec && t0 + 8 <= K) {
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const float4 v = __ldg(reinterpret_cast<const float4*>(src) + q);
-        xr[2 * q] = v.x * s;
-        xi[2 * q] = v.y * s;
-        xr[2 * q + 1] = v.z * s;
-        xi[2 * q + 1] = v.w * s;
-      }
-    } else {
-#pragma unroll
-      for (int b = 0; b < 8; ++b) {
-        const float2 v = (t0 + b < K) ? __ldg(src + b) : make_float2(0.f, 0.f);
-        xr[b] = v.x * s;
-        xi[b] = v.y * s;
-      }
-    }
-    uint32_t hr[2], hi_[2], lr[2], li[2];
-#pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      const float* pr = xr + 4 * q;
-      const float* pi = xi + 4 * q;
-      hr[q] = e4m3x2(pr[0], pr[1]) | (e4m3x2(pr[2], pr[3]) << 16);
-      hi_[q] = e4m3x2(pi[0], pi[1]) | (e4m3x2(pi[2], pi[3]) << 16);
-      if (split) {
-        float dr[4], di[4];
-#pragma unroll
-        for (int b = 0; b < 4; ++b) {
-          dr[b] = pr[b] - e4m3_to_float((hr[q] >> (8 * b)) & 0xFFu);
-          di[b] = pi[b] - e4m3_to_float((hi_[q] >> (8 * b)) & 0xFFu);
-        }
-        lr[q] = e4m3x2(dr[0], dr[1]) | (e4m3x2(dr[2], dr[3]) << 16);
-        li[q] = e4m3x2(di[0], di[1]) | (e4m3x2(di[2], di[3]) << 16);
-      }
-    }
-    uint8_t* dst = z + r * zpitch + t0;
-    *reinterpret_cast<uint2*>(dst) = make_uint2(hr[0], hr[1]);
-    *reinterpret_cast<uint2*>(dst + plane) = make_uint2(hi_[0], hi_[1]);
-    if (split) {
-      *reinterpret_cast<uint2*>(dst + Kp) = make_uint2(lr[0], lr[1]);
-      *reinterpret_cast<uint2*>(dst + plane + Kp) = make_uint2(li[0], li[1]);
-    }
-  }
-}
-
 // L2 policy that makes lines the first to be evicted (for data read for
-// the last time).  The loads that use it allocate in L1 at evict-first
-// priority: a thread's four 16-byte loads of a unit fall into sectors that
-// neighbouring lanes share, and the second load of each sector then hits L1
-// (85.1 against 87.7 us at 8 channels with no L1 allocation).
+// the last time).
 __device__ __forceinline__ uint64_t l2_evict_first_policy() {
   uint64_t pol;
   asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol));
@@ -184,23 +103,115 @@ __device__ __forceinline__ float4 ldg_last_use(const float4* p, uint64_t pol) {
   return v;
 }
 
-// The 8 samples t0 .. t0 + 7 of one row (src = the row + t0) as Re and Im
-// arrays; samples at or past K read as 0.  pol != 0: an L2 policy for the
-// 16-byte loads (the samples' last use).
-__device__ __forceinline__ void load_unit(const float2* __restrict__ src, int t0, int K, bool vec,
+// Half a warp takes a span of 128 samples of one row, in two layouts: loaded,
+// lane h (0..15) holds the samples 32 q + 2 h and 32 q + 2 h + 1 (q < 4), so that
+// each 16-byte load of the half warp covers 256 consecutive bytes; stored, the
+// samples 8 h .. 8 h + 7, 8 bytes of every plane.  (Lanes that loaded their own
+// 8 samples asked for 32 sectors with every load, four times over: 203 against
+// 178 us for 16 channels of 4096 x 1024 in the cooperative kernel.)  src = the row + the span's first sample t0; samples at or past K
+// read as 0.  pol != 0: an L2 policy for the 16-byte loads (the samples' last
+// use).
+__device__ __forceinline__ void load_span(const float2* __restrict__ src, int t0, int K, bool vec,
                                           float (&xr)[8], float (&xi)[8], uint64_t pol = 0) {
-  if (vec && t0 + 8 <= K) {
+  const int h = int(threadIdx.x) & 15;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const float4* p4 = reinterpret_cast<const float4*>(src) + q;
+  for (int q = 0; q < 4; ++q) {
+    const int t = 32 * q + 2 * h;
+    if (vec && t0 + t < K) {  // K is even
+      const float4* p4 = reinterpret_cast<const float4*>(src + t);
       const float4 v = pol ? ldg_last_use(p4, pol) : __ldg(p4);
       xr[2 * q] = v.x, xi[2 * q] = v.y, xr[2 * q + 1] = v.z, xi[2 * q + 1] = v.w;
-    }
-  } else {
+    } else {
 #pragma unroll
-    for (int b = 0; b < 8; ++b) {
-      const float2 v = (t0 + b < K) ? __ldg(src + b) : make_float2(0.f, 0.f);
-      xr[b] = v.x, xi[b] = v.y;
+      for (int b = 0; b < 2; ++b) {
+        const float2 v = t0 + t + b < K ? __ldg(src + t + b) : make_float2(0.f, 0.f);
+        xr[2 * q + b] = v.x, xi[2 * q + b] = v.y;
+      }
+    }
+  }
+}
+
+// The bytes of a span from the loaded to the stored layout: w[q] holds this
+// lane's pair q as Re, Re, Im, Im; re and im receive the 8 bytes of the samples
+// 8 h .. 8 h + 7.  buf: 64 words of shared memory of the half warp.
+__device__ __forceinline__ void span_bytes(const uint32_t (&w)[4], uint32_t* buf, uint2& re,
+                                           uint2& im) {
+  const int h = int(threadIdx.x) & 15;
+  const uint32_t half = 0xFFFFu << (int(threadIdx.x) & 16);
+#pragma unroll
+  for (int q = 0; q < 4; ++q) buf[16 * q + h] = w[q];
+  __syncwarp(half);
+  const uint4 v = *reinterpret_cast<const uint4*>(buf + 4 * h);
+  __syncwarp(half);  // read before the next span is written
+  re = make_uint2(__byte_perm(v.x, v.y, 0x5410), __byte_perm(v.z, v.w, 0x5410));
+  im = make_uint2(__byte_perm(v.x, v.y, 0x7632), __byte_perm(v.z, v.w, 0x7632));
+}
+
+// E4M3 of a span's scaled samples, in the loaded layout (span_bytes).
+__device__ __forceinline__ void span_e4m3(const float (&xr)[8], const float (&xi)[8],
+                                          uint32_t (&w)[4]) {
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+    w[q] = e4m3x2(xr[2 * q], xr[2 * q + 1]) | (e4m3x2(xi[2 * q], xi[2 * q + 1]) << 16);
+}
+
+// A half warp quantises 128 samples of one row (load_span; Kp is a multiple of
+// 128); the thread with a channel's first samples stores its out_scale.  vec
+// (uniform): K even and the input 16-byte aligned.
+__global__ void __launch_bounds__(256) quantize_kernel(const float2* __restrict__ a,
+                                                       uint8_t* __restrict__ z, int64_t rows,
+                                                       int K, int Kp, int zpitch, int n,
+                                                       const uint32_t* __restrict__ amax_bits,
+                                                       float* __restrict__ out_scale, int split,
+                                                       int rows_per_block, int vec) {
+  __shared__ __align__(16) uint32_t bytes[16][64];
+  dev::griddep_wait();  // the channels' amax
+  dev::griddep_launch();
+  const int chunks = Kp >> 3;
+  const int64_t r0 = int64_t(blockIdx.x) * rows_per_block;
+  const int64_t nrows64 = rows - r0 < rows_per_block ? rows - r0 : rows_per_block;
+  const int nloc = int(nrows64) * chunks;  // a multiple of 16: half warps stay together
+  const int64_t plane = rows * int64_t(zpitch);
+  uint32_t* buf = bytes[threadIdx.x >> 4];
+  // the block's rows belong to at most a few channels: 32-bit channel index
+  const int c0 = int(r0 / n), rin0 = int(r0 - int64_t(c0) * n);
+  int cs = -1;  // the channel s belongs to
+  float s = 1.f;
+  for (int l = threadIdx.x; l < nloc; l += blockDim.x) {
+    const int rl = l / chunks;
+    const int t0 = (l - rl * chunks) << 3;  // this lane's samples in the stored layout
+    const int64_t r = r0 + rl;
+    const int c = c0 + (rin0 + rl) / n;
+    if (c != cs) {
+      s = channel_scale(__uint_as_float(__ldg(amax_bits + c)));
+      cs = c;
+    }
+    if (t0 == 0 && r == int64_t(c) * n) out_scale[c] = 1.f / (s * s);
+    const int ts = t0 & ~127;
+    float xr[8], xi[8];
+    load_span(a + r * K + ts, ts, K, vec, xr, xi);
+#pragma unroll
+    for (int b = 0; b < 8; ++b) xr[b] *= s, xi[b] *= s;
+    uint32_t w[4];
+    uint2 re, im;
+    span_e4m3(xr, xi, w);
+    span_bytes(w, buf, re, im);
+    uint8_t* dst = z + r * zpitch + t0;
+    *reinterpret_cast<uint2*>(dst) = re;
+    *reinterpret_cast<uint2*>(dst + plane) = im;
+    if (split) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+#pragma unroll
+        for (int b = 0; b < 2; ++b) {
+          xr[2 * q + b] -= e4m3_to_float((w[q] >> (8 * b)) & 0xFFu);
+          xi[2 * q + b] -= e4m3_to_float((w[q] >> (16 + 8 * b)) & 0xFFu);
+        }
+      }
+      span_e4m3(xr, xi, w);
+      span_bytes(w, buf, re, im);
+      *reinterpret_cast<uint2*>(dst + Kp) = re;
+      *reinterpret_cast<uint2*>(dst + plane + Kp) = im;
     }
   }
 }
@@ -221,10 +232,11 @@ struct UnitWalk {
     col += dcol;
     if (col >= chunks) col -= chunks, ++row;
   }
-  __device__ __forceinline__ int t0() const { return col << 3; }
-  // offsets of the unit's first sample in a channel's input ([n][K]) and
-  // planes (pitch zpitch)
-  __device__ __forceinline__ int64_t offset(int K) const { return int64_t(row) * K + (col << 3); }
+  // first sample of the unit's span (load_span)
+  __device__ __forceinline__ int t0() const { return (col & ~15) << 3; }
+  // offsets of the span's first sample in a channel's input ([n][K]), and of
+  // the unit's in the planes (pitch zpitch)
+  __device__ __forceinline__ int64_t offset(int K) const { return int64_t(row) * K + t0(); }
   __device__ __forceinline__ int64_t zoffset(int zpitch) const {
     return int64_t(row) * zpitch + (col << 3);
   }
@@ -257,24 +269,23 @@ __device__ __forceinline__ float wait_channel_scale(int cq, float* __restrict__ 
   return sc;
 }
 
-// Quantise one unit (8 samples, Re xr / Im xi) with scale sc into the planes
-// at dst (plane 1 at + plane, plane 2 = -plane 0 at + 2 plane when neg), with
-// quantize_kernel's arithmetic; streaming stores (the planes are not read
-// again by this kernel).
+// Quantise one unit's span (load_span) with scale sc into the planes, this
+// lane's 8 samples at dst (plane 1 at + plane, plane 2 = -plane 0 at + 2 plane
+// when neg), with quantize_kernel's arithmetic; streaming stores (the planes
+// are not read again by this kernel).
 __device__ __forceinline__ void quantise_unit(float (&xr)[8], float (&xi)[8], float sc,
-                                              uint8_t* __restrict__ dst, int64_t plane, int neg) {
+                                              uint32_t* buf, uint8_t* __restrict__ dst,
+                                              int64_t plane, int neg) {
 #pragma unroll
   for (int b = 0; b < 8; ++b) xr[b] *= sc, xi[b] *= sc;
-  uint32_t hr[2], hi_[2];
-#pragma unroll
-  for (int q = 0; q < 2; ++q) {
-    hr[q] = e4m3x2(xr[4 * q], xr[4 * q + 1]) | (e4m3x2(xr[4 * q + 2], xr[4 * q + 3]) << 16);
-    hi_[q] = e4m3x2(xi[4 * q], xi[4 * q + 1]) | (e4m3x2(xi[4 * q + 2], xi[4 * q + 3]) << 16);
-  }
+  uint32_t w[4];
+  uint2 re, im;
+  span_e4m3(xr, xi, w);
+  span_bytes(w, buf, re, im);
   constexpr uint32_t kS = 0x80808080u;
-  __stcs(reinterpret_cast<uint2*>(dst), make_uint2(hr[0], hr[1]));
-  __stcs(reinterpret_cast<uint2*>(dst + plane), make_uint2(hi_[0], hi_[1]));
-  if (neg) __stcs(reinterpret_cast<uint2*>(dst + 2 * plane), make_uint2(hr[0] ^ kS, hr[1] ^ kS));
+  __stcs(reinterpret_cast<uint2*>(dst), re);
+  __stcs(reinterpret_cast<uint2*>(dst + plane), im);
+  if (neg) __stcs(reinterpret_cast<uint2*>(dst + 2 * plane), make_uint2(re.x ^ kS, re.y ^ kS));
 }
 
 // Channel amax, scale and quantisation in one cooperative launch (every
@@ -300,11 +311,13 @@ __device__ __forceinline__ void quantise_unit(float (&xr)[8], float (&xi)[8], fl
 // so both give the same bits.
 __global__ void __launch_bounds__(256, 4) scale_quantize_kernel(
     const float2* __restrict__ a, uint8_t* __restrict__ z, int K, int Kp, int zpitch, int n,
-    int batch, int neg, float* __restrict__ out_scale, uint32_t* amax_bits, uint32_t* arrive, uint32_t* status, int vec) {
+    int batch, int neg, float* __restrict__ out_scale, uint32_t* amax_bits, uint32_t* arrive,
+    uint32_t* status, int vec) {
   dev::griddep_launch();
   const int chunks = Kp >> 3;
   const int64_t units = int64_t(n) * chunks;
-  const int64_t per_blk = (units + gridDim.x - 1) / gridDim.x;
+  // whole spans of 16 units per block, so that half warps stay together
+  const int64_t per_blk = ((units + gridDim.x - 1) / gridDim.x + 15) / 16 * 16;
   const int64_t u0 = int64_t(blockIdx.x) * per_blk;
   const int len = u1_len(u0, per_blk, units);
   const int t = int(threadIdx.x), bd = int(blockDim.x);
@@ -315,6 +328,8 @@ __global__ void __launch_bounds__(256, 4) scale_quantize_kernel(
   const uint64_t pol = l2_evict_first_policy();  // channel c - 1's samples: read for the last time
   __shared__ float wm[2][8];
   __shared__ float s_scale[2];
+  __shared__ __align__(16) uint32_t bytes[16][64];
+  uint32_t* buf = bytes[threadIdx.x >> 4];
   bool aborted = false;  // thread 0's
   for (int c = 0; c <= batch; ++c) {
     const bool amax_step = c < batch, quant_step = c >= 1;
@@ -336,15 +351,15 @@ __global__ void __launch_bounds__(256, 4) scale_quantize_kernel(
       for (; ka + 1 < kend; ka += 2) {
         UnitWalk w2 = wa;
         w2.next();
-        load_unit(cur + wa.offset(K), wa.t0(), K, vec, xr, xi);
-        load_unit(cur + w2.offset(K), w2.t0(), K, vec, yr, yi);
+        load_span(cur + wa.offset(K), wa.t0(), K, vec, xr, xi);
+        load_span(cur + w2.offset(K), w2.t0(), K, vec, yr, yi);
         amax_of(xr, xi);
         amax_of(yr, yi);
         w2.next();
         wa = w2;
       }
       if (ka < kend) {
-        load_unit(cur + wa.offset(K), wa.t0(), K, vec, xr, xi);
+        load_span(cur + wa.offset(K), wa.t0(), K, vec, xr, xi);
         amax_of(xr, xi);
         wa.next();
         ++ka;
@@ -358,10 +373,10 @@ __global__ void __launch_bounds__(256, 4) scale_quantize_kernel(
       sc = s_scale[par];
       if (amax_step) {  // 3
         for (; ka < cnt; ++ka, ++kb) {
-          load_unit(cur + wa.offset(K), wa.t0(), K, vec, xr, xi);
-          load_unit(prev + wb.offset(K), wb.t0(), K, vec, yr, yi, pol);
+          load_span(cur + wa.offset(K), wa.t0(), K, vec, xr, xi);
+          load_span(prev + wb.offset(K), wb.t0(), K, vec, yr, yi, pol);
           amax_of(xr, xi);
-          quantise_unit(yr, yi, sc, zprev + wb.zoffset(zpitch), plane, neg);
+          quantise_unit(yr, yi, sc, buf, zprev + wb.zoffset(zpitch), plane, neg);
           wa.next();
           wb.next();
         }
@@ -383,16 +398,16 @@ __global__ void __launch_bounds__(256, 4) scale_quantize_kernel(
       for (; kb + 1 < cnt; kb += 2) {
         UnitWalk w2 = wb;
         w2.next();
-        load_unit(prev + wb.offset(K), wb.t0(), K, vec, xr, xi, pol);
-        load_unit(prev + w2.offset(K), w2.t0(), K, vec, yr, yi, pol);
-        quantise_unit(xr, xi, sc, zprev + wb.zoffset(zpitch), plane, neg);
-        quantise_unit(yr, yi, sc, zprev + w2.zoffset(zpitch), plane, neg);
+        load_span(prev + wb.offset(K), wb.t0(), K, vec, xr, xi, pol);
+        load_span(prev + w2.offset(K), w2.t0(), K, vec, yr, yi, pol);
+        quantise_unit(xr, xi, sc, buf, zprev + wb.zoffset(zpitch), plane, neg);
+        quantise_unit(yr, yi, sc, buf, zprev + w2.zoffset(zpitch), plane, neg);
         w2.next();
         wb = w2;
       }
       if (kb < cnt) {
-        load_unit(prev + wb.offset(K), wb.t0(), K, vec, xr, xi, pol);
-        quantise_unit(xr, xi, sc, zprev + wb.zoffset(zpitch), plane, neg);
+        load_span(prev + wb.offset(K), wb.t0(), K, vec, xr, xi, pol);
+        quantise_unit(xr, xi, sc, buf, zprev + wb.zoffset(zpitch), plane, neg);
       }
     }
   }
@@ -444,9 +459,10 @@ cudaError_t launch_float_to_planes(const void* a, uint8_t* z, int64_t rows, int 
   // The cooperative kernel takes a step per channel, each with a wait for the
   // whole grid, and saves the second read from HBM: it needs a channel that is
   // long against the wait, or a single one.  Promotion in us, cooperative / two
-  // kernels: 16 channels of 33.6 MB 205 / 231, 4 of them 64 / 72; 8 of 16.8 MB
-  // 76 / 71; 16 of 8.4 MB 70 / 64, of 4.2 MB 54 / 30, of 1.2 MB 47 / 19; one of
-  // 33.6 MB 20 / 22, of 5.6 MB 12 / 14.  The split mode (hi and lo columns) was
+  // kernels: 16 channels of 33.6 MB 178 / 220, 4 of them 56 / 67, one of them
+  // 18.2 / 18.7, one of 5.6 MB 11.7 / 12.1; before either loaded whole spans: 8
+  // channels of 16.8 MB 76 / 71, 16 of 8.4 MB 70 / 64, of 4.2 MB 54 / 30, of 1.2
+  // MB 47 / 19.  The split mode (hi and lo columns) was
   // slower on it at any size: 1.02 against 0.91 ms at 4096 x 64 x 1024.
   const bool large = batch == 1 || int64_t(n) * K * int64_t(sizeof(float2)) >= 24000000;
   const int per_sm = split || !large ? 0 : scale_quantize_blocks_per_sm();
