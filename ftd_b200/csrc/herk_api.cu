@@ -193,16 +193,16 @@ ftdx_status prepare(ftdx_handle h, const HerkCall& c, cudaStream_t s, const Plan
 
 // Strategy of a call on a handle whose user has set none: the single-CTA
 // kernel, with the promotion fused in or not and K split or not, whichever a
-// small model of the device time puts first.  Its terms, in us, fitted to
-// 35 shapes of 1 to 2112 tiles and 2 to 512 k-blocks on 148 SMs (the pick is
-// within 11% of the best split and kernel tried at each, most within 3%):
-//   a tile of b k-blocks takes max(0.75 b, 2.6) + 0.8 -- the MMAs or the
-//     stores, then the pipeline's fill; 1.25 b with the conversion fused in;
-//   the separate promotion 3 for its launch + the planes' bytes at 5.5 TB/s;
-//   split-K 6 for its reduction + the partial triangles at 3 TB/s.
-// 256 inputs x 65536 samples x 4 channels (12 tiles): 408 us unsplit with the
-// promotion apart, 70 us as 12 ranges with it fused in; 128 x 256 x 32: 14.3
-// apart, 10 fused in; 512 x 1024 x 30 (300 tiles): 37.3 apart, 39.3 fused in.
+// small model of the device time puts first.  Its terms, in us, fitted to 54
+// shapes of 1 to 2112 tiles and 2 to 512 k-blocks on 148 SMs (the pick is
+// within 13% of the best split and kernel tried at each, most within 3%):
+//   a tile of b k-blocks takes max(0.58 b, 2.2) + 0.6 -- the MMAs or the
+//     stores, then the pipeline's fill; 0.95 b with the conversion fused in;
+//   the separate promotion 2 for its launch + the planes' bytes at 5.5 TB/s;
+//   split-K 3 for its reduction + the partial triangles at 3 TB/s.
+// 256 inputs x 65536 samples x 4 channels (12 tiles): 333 us unsplit with the
+// promotion apart, 56 us as 12 ranges with it fused in; 128 x 256 x 32: 12.6
+// apart, 8.0 fused in; 1024 x 1024 x 16 (576 tiles): 41.1 apart, 43.5 fused in.
 // The choice depends on sizes and on `fused` alone, so that a call prepared
 // for capture (ftdx_init_herk) finds its plan.
 Strategy auto_strategy(const ftdx_context& h, int N, int K, int batch, bool fused_ok,
@@ -218,9 +218,9 @@ Strategy auto_strategy(const ftdx_context& h, int N, int K, int batch, bool fuse
   for (int sp = 1; sp <= int(most) && (sp == 1 || sp * partial <= 256e6); ++sp) {
     const double b = double((kb + sp - 1) / sp);
     const double rounds = double((tiles * sp + h.sm_count - 1) / h.sm_count);
-    const double sum = sp > 1 ? 6.0 + 0.2 * sp + sp * partial / 3e6 : 0.0;
-    const double apart = 3.0 + planes / 5.5e6 + rounds * (std::max(0.75 * b, 2.6) + 0.8) + sum;
-    const double in_one = rounds * (std::max(1.25 * b, 2.6) + 0.8) + sum;
+    const double sum = sp > 1 ? 3.0 + 0.1 * sp + sp * partial / 3e6 : 0.0;
+    const double apart = 2.0 + planes / 5.5e6 + rounds * (std::max(0.58 * b, 2.2) + 0.6) + sum;
+    const double in_one = rounds * (std::max(0.95 * b, 2.2) + 0.6) + sum;
     const bool f = fused_ok && in_one < apart;
     const double us = f ? in_one : apart;
     if (sp == 1 || us < best_us) {

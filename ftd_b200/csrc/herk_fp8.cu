@@ -337,7 +337,7 @@ __device__ __forceinline__ void store_chunk(Out2* p, float2* pc, int i0, int j, 
 
 // kFused (QC input only): tmZ maps the raw QC bytes [rows][K] instead of the
 // operand planes; the producer loads raw tiles (128 rows x 128 samples, one
-// byte each) into a ring of kRawStages, and four converter warps (warps 10-13)
+// byte each) into a ring of kRawStages, and eight converter warps (warps 10-17)
 // turn each into the E4M3 Re / Im planes of an operand stage in the 128-byte
 // swizzled layout the TMA would have written, then release it to the MMA warp.
 //
@@ -769,7 +769,7 @@ __global__ void __launch_bounds__(kFused ? kFusedThreads : kHerkThreads, 1)
           const int i0 = ib + 32 * c;
           if (i0 + 31 < jw || i0 >= n) continue;  // warp-uniform: nothing to store
           if constexpr (kFused) {
-            // 16 rows at a time: the fused kernel's 448 threads get 128 registers
+            // 16 rows at a time: the fused kernel's 576 threads get 112 registers
 #pragma unroll 1
             for (int hr = 0; hr < 2; ++hr) {
               const int i0h = i0 + 16 * hr;
@@ -815,12 +815,15 @@ __global__ void __launch_bounds__(kFused ? kFusedThreads : kHerkThreads, 1)
   } else if (kFused) {
     // ------------------------------------------------ converter warps (kFused)
     // Per stage: 2048 16-byte chunks (1024 on the diagonal).  Chunk
-    // q * 128 + ct (q < 16) is row q * 16 + (ct >> 3) (rows 128-255 = the i
+    // q * 256 + ct (q < 8) is row q * 32 + (ct >> 3) (rows 128-255 = the i
     // block) and 16-byte column ct & 7; a warp's load covers 4 whole raw rows.
     // In the 128-byte swizzled layout, column c of row r sits at
     // r * 128 + ((c ^ (r & 7)) << 4) of its plane; r & 7 = (ct >> 3) & 7 for
     // every q, so each chunk's source and destination are this thread's base
-    // plus a constant.  All loads of a stage are issued before any convert.
+    // plus a constant.  All loads of a half are issued before any convert.
+    // Four warps, one per scheduler with nothing to hide its latencies, took
+    // 1.08 us per k-block off the diagonal, eight take 1.01 (512 k-blocks, 12
+    // CTAs): what is left is the shared memory's traffic.
     const int ct = threadIdx.x - 32 * (2 + kEpiWarps);
     const int src_t = 16 * ct;
     const int dst_t = (ct >> 3) * 128 + (((ct & 7) ^ ((ct >> 3) & 7)) << 4);
@@ -839,23 +842,24 @@ __global__ void __launch_bounds__(kFused ? kFusedThreads : kHerkThreads, 1)
         }
         const uint8_t* src = smem + (raw_addr(r) - smem0) + src_t;
         uint8_t* dst = smem + (plane_addr(stage, 0) - smem0) + dst_t;
-        // two halves of 8 chunks (the j block's rows, then the i block's)
+        // two halves of 4 chunks (the j block's rows, then the i block's)
+        constexpr int kChunkQ = 1024 / kConvThreads, kChunkStep = 16 * kConvThreads;
 #pragma unroll
         for (int hb = 0; hb < 2; ++hb) {
           if (hb == 1 && diag) break;
-          uint4 v[8];
+          uint4 v[kChunkQ];
 #pragma unroll
-          for (int q = 0; q < 8; ++q)
-            v[q] = *reinterpret_cast<const uint4*>(src + (hb * 8 + q) * 2048);
+          for (int q = 0; q < kChunkQ; ++q)
+            v[q] = *reinterpret_cast<const uint4*>(src + (hb * kChunkQ + q) * kChunkStep);
 #pragma unroll
-          for (int q = 0; q < 8; ++q) {
+          for (int q = 0; q < kChunkQ; ++q) {
             uint4 re, im;
             qc4_to_e4m3(v[q].x, re.x, im.x);
             qc4_to_e4m3(v[q].y, re.y, im.y);
             qc4_to_e4m3(v[q].z, re.z, im.z);
             qc4_to_e4m3(v[q].w, re.w, im.w);
             // rows 0-127: planes 0 / 1 (Re_j / Im_j); 128-255: planes 2 / 3
-            const int off = q * 2048 + hb * 2 * kPlaneBytes;
+            const int off = q * kChunkStep + hb * 2 * kPlaneBytes;
             *reinterpret_cast<uint4*>(dst + off) = re;
             *reinterpret_cast<uint4*>(dst + off + kPlaneBytes) = im;
           }

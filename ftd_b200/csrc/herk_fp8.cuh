@@ -50,7 +50,7 @@ static_assert(kSplitSmem <= 232448, "shared memory per CTA");
 // planes into shared memory, so no operand planes exist in HBM.  Two operand
 // stages and three raw stages (128 A rows + 128 B rows of 128 QC bytes); no
 // bulk-store staging.
-constexpr int kConvWarps = 4;
+constexpr int kConvWarps = 8;
 constexpr int kConvThreads = 32 * kConvWarps;
 constexpr int kFusedThreads = kHerkThreads + kConvThreads;
 constexpr int kFusedStages = 2;
