@@ -24,7 +24,15 @@ namespace {
 
 constexpr int kTK = 128;         // time samples per tile
 constexpr int kTS = 128;         // source bytes (ant, chan, pol) per tile
-constexpr int kTPitch = kTK + 4; // transposed tile row pitch (bytes)
+constexpr int kTPitch = kTK;     // transposed tile row pitch (bytes)
+
+// Byte offset of samples 4 kg .. 4 kg + 3 of source byte s in the transposed
+// tile: 16-byte groups of a row are permuted by the row, so that phase 1 (a
+// warp writes one byte column of eight 16-byte source pieces x four words) and
+// phase 2 (16-byte reads, rows 128 bytes apart) touch every bank once.
+__device__ __forceinline__ int tile_at(int s, int kg) {
+  return s * kTPitch + ((((kg >> 2) ^ (s >> 4) ^ s) & 7) << 4) + ((kg & 3) << 2);
+}
 
 __device__ __forceinline__ void put32(uint8_t* dst, const uint32_t (&w)[8], int nbytes) {
   // nbytes valid bytes of the 32 at dst (any alignment)
@@ -43,12 +51,14 @@ __device__ __forceinline__ void put32(uint8_t* dst, const uint32_t (&w)[8], int 
 
 // [t][ant][chan][pol] source.  Block (x, y, z): source bytes [128 x, +128) of
 // a time slice (S = n_ant*n_chan*n_pol bytes each), samples k in [128 y, +128),
-// time_inner z.  The 128 x 128 byte tile is read with coalesced 4-byte loads
-// along the slice, transposed 4 x 4 in registers into shared memory as
-// [source byte][k], then every (source byte, 32 samples) run is converted and
-// written as 32 contiguous bytes per plane (four threads: one 128-byte line).
-// Eight blocks per SM (32 registers, a few bytes spilled) beat six (40
-// registers, no spill): the kernel is latency- and issue-bound.
+// time_inner z.  The 128 x 128 byte tile is read with 16-byte loads (a warp
+// covers 128 bytes of four samples), transposed 4 x 4 in registers into shared
+// memory as [source byte][k], then every (source byte, 32 samples) run is
+// converted and written as 32 contiguous bytes per plane (four threads: one
+// 128-byte line).  Latency- and issue-bound: with 4-byte loads, four times as
+// many, and 4-byte shared-memory reads it took 54.5 us for 2048 antennas x 16
+// channels x 2 pols x 1024 samples (201 MB), so 43.2; six blocks per SM (40
+// registers instead of 32) make no difference.
 __global__ void __launch_bounds__(256, 8) ftd_tacp_to_planes_kernel(const uint8_t* __restrict__ raw,
                                                                  uint8_t* __restrict__ z,
                                                                  FtdGeom g) {
@@ -59,40 +69,52 @@ __global__ void __launch_bounds__(256, 8) ftd_tacp_to_planes_kernel(const uint8_
   const int k0 = blockIdx.y * kTK;
   const int ti = blockIdx.z;
   const int t = threadIdx.x;
-  const bool wide = (S & 3) == 0 && (reinterpret_cast<uintptr_t>(raw) & 3) == 0;
-  // phase 1: kTK / 4 k-groups x 32 s-groups of 4 x 4 bytes, kTK / 32 per thread
-#pragma unroll
-  for (int rep = 0; rep < kTK / 32; ++rep) {
-    const int blk = t + 256 * rep;
-    const int sg = blk & 31, kg = blk >> 5;  // lanes of a warp: consecutive source words
-    uint32_t w[4];
+  // slices start every S bytes, or at t_stride and z_stride (the XEngine's)
+  const int64_t starts = S | g.t_stride | g.z_stride | int64_t(reinterpret_cast<uintptr_t>(raw));
+  const bool words = (starts & 3) == 0, wide = (starts & 15) == 0;
+  // phase 1: thread t takes the source bytes [16 sg, +16) of the samples
+  // 4 kg .. 4 kg + 3 (8 x 32 pieces): four 16-byte loads, where every slice
+  // starts on a 16-byte boundary, and four 4 x 4 byte transposes
+  {
+    const int sg = t & 7, kg = t >> 3;
+    uint32_t w[4][4];  // [sample][word]: byte b of word x = source byte 16 sg + 4 x + b
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
       const int k = k0 + 4 * kg + r;
-      const int64_t s = s0 + 4 * sg;
-      uint32_t v = 0;
-      if (k < g.K) {
-        const uint8_t* src = raw + (g.t_stride ? int64_t(k) * g.t_stride + ti * g.z_stride
-                                               : (int64_t(k) * g.n_ti + ti) * S) + s;
-        if (wide && s + 4 <= S) {
-          v = __ldg(reinterpret_cast<const uint32_t*>(src));
-        } else {
-          for (int b = 0; b < 4; ++b)
-            if (s + b < S) v |= uint32_t(__ldg(src + b)) << (8 * b);
+      const int64_t s = s0 + 16 * sg;
+      const uint8_t* src = raw + (g.t_stride ? int64_t(k) * g.t_stride + ti * g.z_stride
+                                             : (int64_t(k) * g.n_ti + ti) * S) + s;
+      if (wide && k < g.K && s + 16 <= S) {
+        const uint4 v = __ldg(reinterpret_cast<const uint4*>(src));
+        w[r][0] = v.x, w[r][1] = v.y, w[r][2] = v.z, w[r][3] = v.w;
+      } else {
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+          w[r][x] = 0;
+          if (k >= g.K) continue;
+          if (words && s + 4 * x + 4 <= S) {
+            w[r][x] = __ldg(reinterpret_cast<const uint32_t*>(src) + x);
+          } else {
+#pragma unroll
+            for (int b = 0; b < 4; ++b)
+              if (s + 4 * x + b < S) w[r][x] |= uint32_t(__ldg(src + 4 * x + b)) << (8 * b);
+          }
         }
       }
-      w[r] = v;  // byte b = source s + b at sample k0 + 4 kg + r
     }
-    // transpose: out[b] byte r = w[r] byte b
-    const uint32_t lo01 = __byte_perm(w[0], w[1], 0x5140), hi01 = __byte_perm(w[0], w[1], 0x7362);
-    const uint32_t lo23 = __byte_perm(w[2], w[3], 0x5140), hi23 = __byte_perm(w[2], w[3], 0x7362);
-    const uint32_t o0 = __byte_perm(lo01, lo23, 0x5410), o1 = __byte_perm(lo01, lo23, 0x7632);
-    const uint32_t o2 = __byte_perm(hi01, hi23, 0x5410), o3 = __byte_perm(hi01, hi23, 0x7632);
-    uint8_t* d = tileT + (4 * sg) * kTPitch + 4 * kg;
-    *reinterpret_cast<uint32_t*>(d) = o0;
-    *reinterpret_cast<uint32_t*>(d + kTPitch) = o1;
-    *reinterpret_cast<uint32_t*>(d + 2 * kTPitch) = o2;
-    *reinterpret_cast<uint32_t*>(d + 3 * kTPitch) = o3;
+#pragma unroll
+    for (int x = 0; x < 4; ++x) {
+      // transpose: out[b] byte r = w[r] byte b
+      const uint32_t lo01 = __byte_perm(w[0][x], w[1][x], 0x5140);
+      const uint32_t hi01 = __byte_perm(w[0][x], w[1][x], 0x7362);
+      const uint32_t lo23 = __byte_perm(w[2][x], w[3][x], 0x5140);
+      const uint32_t hi23 = __byte_perm(w[2][x], w[3][x], 0x7362);
+      const int s = 16 * sg + 4 * x;
+      *reinterpret_cast<uint32_t*>(tileT + tile_at(s, kg)) = __byte_perm(lo01, lo23, 0x5410);
+      *reinterpret_cast<uint32_t*>(tileT + tile_at(s + 1, kg)) = __byte_perm(lo01, lo23, 0x7632);
+      *reinterpret_cast<uint32_t*>(tileT + tile_at(s + 2, kg)) = __byte_perm(hi01, hi23, 0x5410);
+      *reinterpret_cast<uint32_t*>(tileT + tile_at(s + 3, kg)) = __byte_perm(hi01, hi23, 0x7632);
+    }
   }
   __syncthreads();
   // phase 2: task -> (source byte sl, samples [32 h, +32)), kTK / 64 per thread
@@ -123,9 +145,11 @@ __global__ void __launch_bounds__(256, 8) ftd_tacp_to_planes_kernel(const uint8_
     if (kb >= kend) continue;
     const int nbytes = kend - kb < 32 ? kend - kb : 32;
     uint32_t q[8];
-    const uint8_t* src = tileT + sl * kTPitch + 32 * h;
 #pragma unroll
-    for (int x = 0; x < 8; ++x) q[x] = *reinterpret_cast<const uint32_t*>(src + 4 * x);
+    for (int x = 0; x < 2; ++x) {
+      const uint4 v = *reinterpret_cast<const uint4*>(tileT + tile_at(sl, 8 * h + 4 * x));
+      q[4 * x] = v.x, q[4 * x + 1] = v.y, q[4 * x + 2] = v.z, q[4 * x + 3] = v.w;
+    }
     uint32_t re[8], im[8];
     if (g.twos) {
 #pragma unroll
