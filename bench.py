@@ -996,6 +996,7 @@ def run_splitk_leg(torch, dev, N=256, K=65536, B=4, seed=10):
     C = torch.empty(B, tri_size(N), 2, device=dev)
     flops = herk_flops(N, K, B)
     with Correlator(device=dev.index) as c:
+        c.set_strategy(0, 0)  # one CTA per tile over all of K
         plain = _timed(torch, lambda: c.herk(qc, C, N, K, B, input=IN_INT4, output=OUT_FP32,
                                              tune=False), reps=10)
         c.tune(qc, C, N, K, B)

@@ -426,6 +426,12 @@ ftdx_status run_tune(ftdx_handle h, const HerkCall& c, cudaStream_t s, TuneEntry
     for (int sp : {2, 4, 8, 16, 32})
       if (sp <= kblocks && plan->num_tiles * (sp / 2) < 2 * h->sm_count)
         cands.push_back(Strategy{0, h->sm_count, sp});
+  // what an untuned call would take, where that is no candidate yet (256 x
+  // 65536 x 4: 91 us as eight ranges with the promotion apart, 66 as twelve with
+  // it fused in)
+  const Strategy untuned = auto_strategy(*h, c.N, c.K, c.batch, fused_ok(c),
+                                         !c.comp && c.out_format == 0);
+  if (!is_fp4(c) && untuned.splits > 1) cands.push_back(untuned);
   st = tune_sweep(
       h, [&](const Strategy& cand, cudaStream_t ss) { return launch_all(h, c, cand, ss); },
       cands, s, &best);
