@@ -111,6 +111,8 @@ struct HerkArgs {
   // K segments: segment s pairs the A (j) operand's k-blocks seg_a[s] + kk
   // with the B (i) operand's k-blocks seg_b[s] + kk, kk < kblocks, all
   // accumulated into one result (nseg = 1, offsets 0: a plain HERK).
+  // The single-CTA kernel takes nseg = 3 as hi hi + hi lo + lo hi with the lo
+  // columns seg_b[1] k-blocks after the hi ones.
   int32_t nseg;
   int32_t seg_a[3];
   int32_t seg_b[3];
