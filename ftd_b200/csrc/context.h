@@ -15,6 +15,7 @@
 
 #include "../../include/ftdx.h"
 #include "herk_fp8.cuh"
+#include "strategy.h"
 
 namespace ftdx {
 
@@ -25,26 +26,6 @@ struct Plan {
   int num_tiles = 0;
   int num_chans = 0;
   ~Plan();
-};
-
-constexpr int kStoreFp6 = 4;
-constexpr int kStoreS8 = 8;   // with store mode 2: signed 8-bit operands, kind::i8 MMAs
-constexpr int kStoreFused = 16;  // alone (mode 0 + 16): QC promotion fused into the single-CTA kernel
-// Launch strategy of the correlator kernel; chosen by the autotuner.
-struct Strategy {
-  // 0: direct stores, 1: shared-memory staging + bulk copies,
-  // 2: CTA-pair kernel (256 x 128 tiles on two SMs, direct stores);
-  // 3: CTA-pair kernel with bulk-copy stores for interior tiles;
-  // + kStoreFp6: operands as packed FP6 E3M2 planes (QC input, exact);
-  // + kStoreS8 (pair only): signed 8-bit planes, integer MMAs (QC input, exact)
-  // kStoreFused (alone): single CTA, direct stores, the QC bytes converted to
-  // E4M3 inside the correlator (uniform INT4 calls; others run as 0)
-  int store_mode = 0;
-  int grid = 0;        // persistent CTAs (0: one per SM); -1: one CTA per tile (not persistent)
-  int splits = 1;      // split-K: K is cut into this many ranges, partials summed afterwards
-  bool operator==(const Strategy& o) const {
-    return store_mode == o.store_mode && grid == o.grid && splits == o.splits;
-  }
 };
 
 // Autotune cache key: device, problem shape and precisions.
@@ -96,9 +77,7 @@ struct ftdx_context {
   uint8_t* aux = nullptr;
   size_t aux_cap = 0;
   uint32_t* d_status = nullptr;
-  // split-K partial triangles (grown on demand)
-  uint8_t* split_ws = nullptr;
-  size_t split_ws_cap = 0;
+  ftdx::Partials partials;  // split-K partial triangles
   // stridedBatchGEMM's FP16 staging (narrowed input, FP16 triangles), grown on demand
   uint8_t* strided_ws = nullptr;
   size_t strided_ws_cap = 0;
@@ -143,7 +122,7 @@ ftdx_status ensure_aux(ftdx_handle h, size_t bytes, cudaStream_t s);
 // column inputs c and ti over 128 row inputs r <= c
 ftdx_status get_plan(ftdx_handle h, int N, int kblocks, int batch, cudaStream_t s,
                      const Plan** out, bool pair = false, int splits = 1, bool upper = false);
-ftdx_status ensure_split_ws(ftdx_handle h, size_t bytes, cudaStream_t s);
+ftdx_status ensure_partials(ftdx_handle h, size_t bytes, cudaStream_t s);
 // fp6: planes of packed E3M2 codes (the kernels' fp6 operand form)
 ftdx_status encode_planes_map(ftdx_handle h, uint8_t* z, int64_t rows, int64_t Kp,
                               CUtensorMap* tm, int box_rows = kTile, int nplanes = 2,

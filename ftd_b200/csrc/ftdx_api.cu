@@ -116,24 +116,27 @@ ftdx_status ensure_workspace(ftdx_handle h, size_t bytes, cudaStream_t s) {
   return FTDX_OK;
 }
 
-ftdx_status ensure_split_ws(ftdx_handle h, size_t bytes, cudaStream_t s) {
-  if (bytes <= h->split_ws_cap) return FTDX_OK;
+ftdx_status ensure_partials(ftdx_handle h, size_t bytes, cudaStream_t s) {
+  if (bytes <= h->partials.cap) return FTDX_OK;
   if (stream_capturing(s))
     return fail(h, FTDX_ERR_CAPACITY, "split-K workspace needed while capturing; call once first");
-  if (h->split_ws) {
-    cudaDeviceSynchronize();
-    cudaFree(h->split_ws);
-    h->split_ws = nullptr;
-    h->split_ws_cap = 0;
-    release_graphs(h);
-  }
-  cudaError_t e = cudaMalloc(&h->split_ws, bytes);
-  if (e != cudaSuccess) {
-    cudaGetLastError();
+  cudaError_t e = cudaSuccess;
+  const bool ok = h->partials.grow(
+      bytes,
+      [&](size_t n) {
+        void* p = nullptr;
+        e = cudaMalloc(&p, n);
+        if (e != cudaSuccess) cudaGetLastError();
+        return e == cudaSuccess ? static_cast<uint8_t*>(p) : nullptr;
+      },
+      [&](uint8_t* p) {
+        cudaDeviceSynchronize();
+        cudaFree(p);
+        release_graphs(h);
+      });
+  if (!ok)
     return fail(h, FTDX_ERR_ALLOC, "cudaMalloc(%zu) for split-K partials: %s", bytes,
                 cudaGetErrorString(e));
-  }
-  h->split_ws_cap = bytes;
   return FTDX_OK;
 }
 
@@ -375,7 +378,7 @@ ftdx_status ftdx_destroy(ftdx_handle h) {
   for (auto e : h->event_pool) cudaEventDestroy(e);
   if (h->z) cudaFree(h->z);
   if (h->aux) cudaFree(h->aux);
-  if (h->split_ws) cudaFree(h->split_ws);
+  h->partials.release([](uint8_t* p) { cudaFree(p); });
   if (h->strided_ws) cudaFree(h->strided_ws);
   if (h->d_status) cudaFree(h->d_status);
   if (h->capture_stream) cudaStreamDestroy(h->capture_stream);

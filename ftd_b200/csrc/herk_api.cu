@@ -184,51 +184,10 @@ ftdx_status prepare(ftdx_handle h, const HerkCall& c, cudaStream_t s, const Plan
     if (st != FTDX_OK) return st;
   }
   if (splits > 1) {
-    st = ensure_split_ws(h, size_t(splits) * size_t(c.batch) *
-                                size_t(int64_t(c.N) * (c.N + 1) / 2) * sizeof(float2), s);
+    st = ensure_partials(h, split_bytes(c.N, c.batch, splits), s);
     if (st != FTDX_OK) return st;
   }
   return get_plan(h, c.N, int(Kp / kStageK), c.batch, s, plan, pair, splits, c.out_format == 1);
-}
-
-// Strategy of a call on a handle whose user has set none: the single-CTA
-// kernel, with the promotion fused in or not and K split or not, whichever a
-// small model of the device time puts first.  Its terms, in us, fitted to 54
-// shapes of 1 to 2112 tiles and 2 to 512 k-blocks on 148 SMs (the pick is
-// within 13% of the best split and kernel tried at each, most within 3%):
-//   a tile of b k-blocks takes max(0.58 b, 2.2) + 0.6 -- the MMAs or the
-//     stores, then the pipeline's fill; 0.95 b with the conversion fused in;
-//   the separate promotion 2 for its launch + the planes' bytes at 5.5 TB/s;
-//   split-K 3 for its reduction + the partial triangles at 3 TB/s.
-// 256 inputs x 65536 samples x 4 channels (12 tiles): 333 us unsplit with the
-// promotion apart, 56 us as 12 ranges with it fused in; 128 x 256 x 32: 12.6
-// apart, 8.0 fused in; 1024 x 1024 x 16 (576 tiles): 41.1 apart, 43.5 fused in.
-// The choice depends on sizes and on `fused` alone, so that a call prepared
-// for capture (ftdx_init_herk) finds its plan.
-Strategy auto_strategy(const ftdx_context& h, int N, int K, int batch, bool fused_ok,
-                       bool split_ok) {
-  const int64_t nb = (N + kTile - 1) / kTile, tiles = nb * (nb + 1) / 2 * batch;
-  const int64_t kb = round_up(K, kStageK) / kStageK;
-  const double planes = 3.0 * N * double(batch) * double(kb * kStageK);
-  const double partial = 4.0 * N * (N + 1.0) * batch;  // bytes of one split's triangles
-  Strategy best;
-  // past eight tiles per SM the last round costs little and partials much
-  const int64_t most = split_ok && tiles <= 8 * h.sm_count ? std::min<int64_t>(32, kb) : 1;
-  double best_us = 0;
-  for (int sp = 1; sp <= int(most) && (sp == 1 || sp * partial <= 256e6); ++sp) {
-    const double b = double((kb + sp - 1) / sp);
-    const double rounds = double((tiles * sp + h.sm_count - 1) / h.sm_count);
-    const double sum = sp > 1 ? 3.0 + 0.1 * sp + sp * partial / 3e6 : 0.0;
-    const double apart = 2.0 + planes / 5.5e6 + rounds * (std::max(0.58 * b, 2.2) + 0.6) + sum;
-    const double in_one = rounds * (std::max(0.95 * b, 2.2) + 0.6) + sum;
-    const bool f = fused_ok && in_one < apart;
-    const double us = f ? in_one : apart;
-    if (sp == 1 || us < best_us) {
-      best = Strategy{f ? kStoreFused : 0, 0, sp};
-      best_us = us;
-    }
-  }
-  return best;
 }
 
 // NVFP4: the CTA pair from four rounds of its tiles on, where the operand
@@ -246,7 +205,7 @@ Strategy fp4_strategy(int N, int K, int batch) {
 Strategy untuned_strategy(ftdx_handle h, const HerkCall& c) {
   if (h->user_strategy) return h->default_strategy;
   if (is_fp4(c)) return fp4_strategy(c.N, c.K, c.batch);
-  return auto_strategy(*h, c.N, c.K, c.batch, fused_ok(c), !c.comp && c.out_format == 0);
+  return auto_strategy(h->sm_count, c.N, c.K, c.batch, fused_ok(c), !c.comp && c.out_format == 0);
 }
 
 // Before an untuned call: everything that calls of its shape may need under a
@@ -259,7 +218,7 @@ ftdx_status prepare_auto(ftdx_handle h, const HerkCall& c, cudaStream_t s, Strat
   const Plan* plan = nullptr;
   ftdx_status st = prepare(h, c, s, &plan);
   for (int f = 0; f < 2 && st == FTDX_OK; ++f) {
-    const Strategy a = auto_strategy(*h, c.N, c.K, c.batch, f == 1, true);
+    const Strategy a = auto_strategy(h->sm_count, c.N, c.K, c.batch, f == 1, true);
     if (a.splits <= 1) continue;
     st = prepare(h, c, s, &plan, false, a.splits);
     if (st == FTDX_ERR_ALLOC) {
@@ -356,7 +315,9 @@ ftdx_status launch_all(ftdx_handle h, const HerkCall& c, const Strategy& strat, 
     args.out2 = c.comp;
   }
   if (splits > 1) {  // partial triangles, reduced below
-    args.out = h->split_ws;
+    args.out = h->partials.ptr;
+    // the handle's own graphs are dropped with the buffer, a caller's cannot be
+    if (s != h->capture_stream && stream_capturing(s)) h->partials.captured = true;
     args.out_fp16 = 0;
     args.alpha = 1.f;
     args.beta = 0.f;
@@ -383,7 +344,7 @@ ftdx_status launch_all(ftdx_handle h, const HerkCall& c, const Strategy& strat, 
   }
   if (e != cudaSuccess) return cuda_fail(h, e, "correlator kernel launch");
   if (splits > 1) {
-    e = launch_split_reduce(reinterpret_cast<const float2*>(h->split_ws), c.C,
+    e = launch_split_reduce(reinterpret_cast<const float2*>(h->partials.ptr), c.C,
                             c.output == FTDX_OUT_FP16 ? 1 : 0, int64_t(c.N) * (c.N + 1) / 2,
                             c.batch, splits, c.alpha, c.beta,
                             c.input == FTDX_IN_FP32 ? out_scale : nullptr, h->sm_count, s);
@@ -429,7 +390,7 @@ ftdx_status run_tune(ftdx_handle h, const HerkCall& c, cudaStream_t s, TuneEntry
   // what an untuned call would take, where that is no candidate yet (256 x
   // 65536 x 4: 91 us as eight ranges with the promotion apart, 66 as twelve with
   // it fused in)
-  const Strategy untuned = auto_strategy(*h, c.N, c.K, c.batch, fused_ok(c),
+  const Strategy untuned = auto_strategy(h->sm_count, c.N, c.K, c.batch, fused_ok(c),
                                          !c.comp && c.out_format == 0);
   if (!is_fp4(c) && untuned.splits > 1) cands.push_back(untuned);
   st = tune_sweep(
@@ -682,8 +643,12 @@ ftdx_status ftdx_init_herk(ftdx_handle h, int N, int K, int batch, void* stream)
                    FTDX_IN_INT4, FTDX_OUT_FP32, 1.f, 0.f};
   const Plan* p = nullptr;
   Strategy strat;
-  if (!h->user_strategy && !stream_capturing(static_cast<cudaStream_t>(stream)))
+  if (!h->user_strategy && !stream_capturing(static_cast<cudaStream_t>(stream))) {
+    // partial triangles for every shape up to this one; where they do not fit,
+    // for this one (below)
+    ensure_partials(h, most_split_bytes(N, K, batch), static_cast<cudaStream_t>(stream));
     return prepare_auto(h, c, static_cast<cudaStream_t>(stream), &strat);
+  }
   return prepare(h, c, static_cast<cudaStream_t>(stream), &p, use_pair(h, h->default_strategy));
 }
 

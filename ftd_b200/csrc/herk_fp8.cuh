@@ -21,10 +21,10 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include "strategy.h"
+
 namespace ftdx {
 
-constexpr int kTile = 128;                   // antennas per operand tile (M = N = 128)
-constexpr int kStageK = 128;                 // samples per pipeline stage (= bytes per plane row)
 constexpr int kPlaneBytes = kTile * kStageK; // 16 KB
 constexpr int kStageBytes = 4 * kPlaneBytes; // A_re, A_im, B_re, B_im
 constexpr int kStages = 3;

@@ -1,0 +1,138 @@
+// strategy.h -- the launch strategy of a correlator call, the rule that picks it
+// where the user has set none, and the device memory that split-K needs.  Host
+// code without CUDA headers.
+#pragma once
+#include <algorithm>
+#include <cstddef>
+#include <cstdint>
+#include <vector>
+
+namespace ftdx {
+
+constexpr int kTile = 128;    // antennas per operand tile (M = N = 128)
+constexpr int kStageK = 128;  // samples per pipeline stage (= bytes per plane row)
+
+constexpr int kStoreFp6 = 4;
+constexpr int kStoreS8 = 8;   // with store mode 2: signed 8-bit operands, kind::i8 MMAs
+constexpr int kStoreFused = 16;  // alone (mode 0 + 16): QC promotion fused into the single-CTA kernel
+// Launch strategy of the correlator kernel; chosen by the autotuner.
+struct Strategy {
+  // 0: direct stores, 1: shared-memory staging + bulk copies,
+  // 2: CTA-pair kernel (256 x 128 tiles on two SMs, direct stores);
+  // 3: CTA-pair kernel with bulk-copy stores for interior tiles;
+  // + kStoreFp6: operands as packed FP6 E3M2 planes (QC input, exact);
+  // + kStoreS8 (pair only): signed 8-bit planes, integer MMAs (QC input, exact)
+  // kStoreFused (alone): single CTA, direct stores, the QC bytes converted to
+  // E4M3 inside the correlator (uniform INT4 calls; others run as 0)
+  int store_mode = 0;
+  int grid = 0;        // persistent CTAs (0: one per SM); -1: one CTA per tile (not persistent)
+  int splits = 1;      // split-K: K is cut into this many ranges, partials summed afterwards
+  bool operator==(const Strategy& o) const {
+    return store_mode == o.store_mode && grid == o.grid && splits == o.splits;
+  }
+};
+
+// Split-K: the most ranges, and the most bytes of partial triangles that the
+// rule below takes.
+constexpr int kMostSplits = 32;
+constexpr size_t kMostSplitBytes = 256000000;
+inline size_t split_bytes(int N, int batch, int splits) {
+  return size_t(splits) * size_t(batch) * size_t(int64_t(N) * (N + 1) / 2) * 8;
+}
+
+// Strategy of a call on a handle whose user has set none: the single-CTA
+// kernel, with the promotion fused in or not and K split or not, whichever a
+// small model of the device time puts first.  Its terms, in us, fitted to 54
+// shapes of 1 to 2112 tiles and 2 to 512 k-blocks on 148 SMs (the pick is
+// within 13% of the best split and kernel tried at each, most within 3%):
+//   a tile of b k-blocks takes max(0.58 b, 2.2) + 0.6 -- the MMAs or the
+//     stores, then the pipeline's fill; 0.95 b with the conversion fused in;
+//   the separate promotion 2 for its launch + the planes' bytes at 5.5 TB/s;
+//   split-K 3 for its reduction + the partial triangles at 3 TB/s.
+// 256 inputs x 65536 samples x 4 channels (12 tiles): 333 us unsplit with the
+// promotion apart, 56 us as 12 ranges with it fused in; 128 x 256 x 32: 12.6
+// apart, 8.0 fused in; 1024 x 1024 x 16 (576 tiles): 41.1 apart, 43.5 fused in.
+// The choice depends on sizes and on `fused` alone, so that a call prepared
+// for capture (ftdx_init_herk) finds its plan.
+inline Strategy auto_strategy(int sm_count, int N, int K, int batch, bool fused_ok,
+                              bool split_ok) {
+  const int64_t nb = (N + kTile - 1) / kTile, tiles = nb * (nb + 1) / 2 * batch;
+  const int64_t kb = (int64_t(K) + kStageK - 1) / kStageK;
+  const double planes = 3.0 * N * double(batch) * double(kb * kStageK);
+  const double partial = double(split_bytes(N, batch, 1));
+  Strategy best;
+  // past eight tiles per SM the last round costs little and partials much
+  const int64_t most = split_ok && tiles <= 8 * sm_count ? std::min<int64_t>(kMostSplits, kb) : 1;
+  double best_us = 0;
+  for (int sp = 1; sp <= int(most) && (sp == 1 || sp * partial <= kMostSplitBytes); ++sp) {
+    const double b = double((kb + sp - 1) / sp);
+    const double rounds = double((tiles * sp + sm_count - 1) / sm_count);
+    const double sum = sp > 1 ? 3.0 + 0.1 * sp + sp * partial / 3e6 : 0.0;
+    const double apart = 2.0 + planes / 5.5e6 + rounds * (std::max(0.58 * b, 2.2) + 0.6) + sum;
+    const double in_one = rounds * (std::max(0.95 * b, 2.2) + 0.6) + sum;
+    const bool f = fused_ok && in_one < apart;
+    const double us = f ? in_one : apart;
+    if (sp == 1 || us < best_us) {
+      best = Strategy{f ? kStoreFused : 0, 0, sp};
+      best_us = us;
+    }
+  }
+  return best;
+}
+
+// The most bytes of partial triangles that auto_strategy takes for any shape up
+// to (N, K, batch).  A smaller shape can take more than a larger one: on 148 SMs
+// 512 inputs x 8192 samples take three ranges for 4 channels (12.6 MB) and seven
+// for 2 (14.7 MB).
+inline size_t most_split_bytes(int N, int K, int batch) {
+  const int64_t kb = (int64_t(K) + kStageK - 1) / kStageK;
+  const int sp = int(std::min<int64_t>(kMostSplits, kb));
+  return sp > 1 ? std::min(kMostSplitBytes, split_bytes(N, batch, sp)) : 0;
+}
+
+// Device memory of the partial triangles, grown on demand.  A buffer that a
+// caller's graph was captured with is not freed when a larger one replaces it,
+// since every replay of that graph writes to it: it stays until release().
+struct Partials {
+  uint8_t* ptr = nullptr;
+  size_t cap = 0;
+  bool captured = false;       // a caller's capture holds ptr
+  std::vector<uint8_t*> held;  // replaced buffers that captures hold
+
+  // alloc(bytes) returns nullptr on failure; drop(p) waits for p's users and
+  // frees it.  False: not enough memory.
+  template <typename Alloc, typename Drop>
+  bool grow(size_t bytes, Alloc alloc, Drop drop) {
+    if (bytes <= cap) return true;
+    uint8_t* p = nullptr;
+    if (captured) {
+      // half as large again, so that all that is held stays below twice the
+      // last buffer, whatever the order of calls and captures
+      size_t n = std::max(bytes, cap + cap / 2);
+      p = alloc(n);
+      if (!p && n > bytes) p = alloc(n = bytes);
+      if (!p) return false;
+      held.push_back(ptr);
+      bytes = n;
+    } else {
+      if (ptr) drop(ptr);
+      ptr = nullptr;
+      cap = 0;
+      p = alloc(bytes);
+      if (!p) return false;
+    }
+    ptr = p;
+    cap = bytes;
+    captured = false;
+    return true;
+  }
+
+  template <typename Free>
+  void release(Free free) {
+    if (ptr) free(ptr);
+    for (uint8_t* p : held) free(p);
+    *this = Partials{};
+  }
+};
+
+}  // namespace ftdx

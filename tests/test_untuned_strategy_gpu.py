@@ -91,3 +91,38 @@ def test_capture(prepare, offset):
         assert np.array_equal(S.cpu().numpy(), ref)
         assert c.device_status() == 0
         del g
+
+
+@pytest.mark.parametrize("init", [True, False])
+def test_graph_outlives_later_calls(init):
+    # a smaller shape takes more partial triangles (seven ranges of 2 channels
+    # against three of 4): the caller's graph keeps the buffer it was captured with.
+    # None of the later calls needs more operand planes than the captured one.
+    N, K, B = 512, 8192, 4
+    qc = oracle.gaussian_qc(21, B, N, K)
+    d = device_bytes(qc)
+    C = torch.full((B, tri_size(N), 2), float("nan"), device=DEV)
+    s = torch.cuda.Stream()
+    with Correlator() as c:
+        if init:
+            c.init_herk(N, K, B)
+        else:
+            c.herk(d, C, N, K, B, input=IN_INT4, output=OUT_FP32, tune=False)
+        torch.cuda.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=s):
+            c.herk(d, C, N, K, B, input=IN_INT4, output=OUT_FP32, tune=False, stream=s)
+        for n, k, b in ((512, 8192, 2), (256, 32768, 2), (700, 8192, 2)):
+            small = oracle.gaussian_qc(n + b, b, n, k)
+            out = torch.full((b, tri_size(n), 2), float("nan"), device=DEV)
+            c.herk(device_bytes(small), out, n, k, b, input=IN_INT4, output=OUT_FP32, tune=False)
+            rows = oracle.herk_qc_rows(small, n, k, b - 1, n - 4, n).astype(np.float32)
+            assert np.array_equal(out[b - 1, tri_size(n - 4):].cpu().numpy(), rows)
+        C.fill_(float("nan"))
+        keep = [torch.full((8 << 20,), 7.0, device=DEV) for _ in range(8)]  # what was freed is reused
+        g.replay()
+        torch.cuda.synchronize()
+        assert np.array_equal(C.cpu().numpy(), oracle.herk_qc(qc, N, K, B).astype(np.float32))
+        assert all(bool((t == 7.0).all()) for t in keep)
+        assert c.device_status() == 0
+        del g
