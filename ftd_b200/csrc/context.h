@@ -122,6 +122,8 @@ ftdx_status ensure_aux(ftdx_handle h, size_t bytes, cudaStream_t s);
 // column inputs c and ti over 128 row inputs r <= c
 ftdx_status get_plan(ftdx_handle h, int N, int kblocks, int batch, cudaStream_t s,
                      const Plan** out, bool pair = false, int splits = 1, bool upper = false);
+// Whether get_plan would find the single-CTA plan of a packed triangle.
+bool have_plan(ftdx_handle h, int N, int kblocks, int batch, int splits);
 ftdx_status ensure_partials(ftdx_handle h, size_t bytes, cudaStream_t s);
 // fp6: planes of packed E3M2 codes (the kernels' fp6 operand form)
 ftdx_status encode_planes_map(ftdx_handle h, uint8_t* z, int64_t rows, int64_t Kp,

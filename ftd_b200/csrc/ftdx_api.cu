@@ -161,16 +161,24 @@ ftdx_status ensure_aux(ftdx_handle h, size_t bytes, cudaStream_t s) {
   return FTDX_OK;
 }
 
+// kblocks < 2^23 (K <= 2^30) and splits <= 32, so pair, split-K and upper-format
+// pair plans never share a key with others
+static std::tuple<int, int, int> plan_key(int N, int kblocks, int batch, bool pair, int splits,
+                                          bool upper) {
+  return std::make_tuple(
+      N, kblocks + (pair ? (1 << 24) : 0) + ((splits - 1) << 25) + (upper ? (1 << 30) : 0), batch);
+}
+
+bool have_plan(ftdx_handle h, int N, int kblocks, int batch, int splits) {
+  return h->plans.count(plan_key(N, kblocks, batch, false, splits, false)) != 0;
+}
+
 // Lower-triangle tile list for `batch` channels of N inputs, channel-major so
 // that concurrently running CTAs share a channel's operand in L2.
 ftdx_status get_plan(ftdx_handle h, int N, int kblocks, int batch, cudaStream_t s,
                      const Plan** out, bool pair, int splits, bool upper) {
   upper = upper && pair;
-  // kblocks < 2^23 (K <= 2^30) and splits <= 32, so pair, split-K and
-  // upper-format pair plans never share a key with others
-  auto key = std::make_tuple(N, kblocks + (pair ? (1 << 24) : 0) + ((splits - 1) << 25) +
-                                    (upper ? (1 << 30) : 0),
-                             batch);
+  const auto key = plan_key(N, kblocks, batch, pair, splits, upper);
   auto it = h->plans.find(key);
   if (it != h->plans.end()) {
     *out = it->second.get();

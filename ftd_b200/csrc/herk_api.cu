@@ -211,21 +211,32 @@ Strategy untuned_strategy(ftdx_handle h, const HerkCall& c) {
 // Before an untuned call: everything that calls of its shape may need under a
 // later capture, whatever their input's alignment or entry point -- two
 // planes, and the tile plans and partial triangles of the strategies that
-// auto_strategy picks.  Where the partial triangles do not fit, *strat
-// becomes the unsplit kernel.
+// auto_strategy picks.  *strat becomes the strategy to run: the rule's, or the
+// unsplit kernel where the partial triangles of the rule's do not fit or, under
+// a capture, are not there.
 ftdx_status prepare_auto(ftdx_handle h, const HerkCall& c, cudaStream_t s, Strategy* strat) {
-  if (h->user_strategy || is_fp4(c) || stream_capturing(s)) return FTDX_OK;
+  if (h->user_strategy || is_fp4(c)) return FTDX_OK;
+  const bool capturing = stream_capturing(s);
+  const bool split_ok = !c.comp && c.out_format == 0;
   const Plan* plan = nullptr;
-  ftdx_status st = prepare(h, c, s, &plan);
-  for (int f = 0; f < 2 && st == FTDX_OK; ++f) {
-    const Strategy a = auto_strategy(h->sm_count, c.N, c.K, c.batch, f == 1, true);
-    if (a.splits <= 1) continue;
-    st = prepare(h, c, s, &plan, false, a.splits);
-    if (st == FTDX_ERR_ALLOC) {
-      *strat = Strategy{};
-      return FTDX_OK;
-    }
+  ftdx_status st = capturing ? FTDX_OK : prepare(h, c, s, &plan);
+  auto have = [&](int splits) {
+    const size_t bytes = split_bytes(c.N, c.batch, splits);
+    if (capturing)
+      return bytes <= h->partials.cap &&
+             have_plan(h, c.N, int(round_up(c.K, kStageK) / kStageK), c.batch, splits);
+    if (h->partials.hopeless(bytes)) return false;
+    const ftdx_status r = prepare(h, c, s, &plan, false, splits);
+    if (r != FTDX_OK && r != FTDX_ERR_ALLOC) st = r;
+    return r == FTDX_OK;
+  };
+  const bool fused = fused_ok(c);
+  if (st == FTDX_OK && !capturing) {  // the other promotion's ranges, before this call's
+    const Strategy o = auto_strategy(h->sm_count, c.N, c.K, c.batch, !fused, split_ok);
+    if (o.splits > 1) have(o.splits);
   }
+  if (st == FTDX_OK)
+    *strat = untuned_choice(h->sm_count, c.N, c.K, c.batch, fused, split_ok, have);
   return st;
 }
 
@@ -393,6 +404,17 @@ ftdx_status run_tune(ftdx_handle h, const HerkCall& c, cudaStream_t s, TuneEntry
   const Strategy untuned = auto_strategy(h->sm_count, c.N, c.K, c.batch, fused_ok(c),
                                          !c.comp && c.out_format == 0);
   if (!is_fp4(c) && untuned.splits > 1) cands.push_back(untuned);
+  // a candidate whose planes or partial triangles do not fit is not one
+  for (size_t i = 1; !is_fp4(c) && i < cands.size();) {
+    const Plan* p = nullptr;
+    st = prepare(h, c, s, &p, use_pair(h, cands[i]), effective_splits(c, cands[i]),
+                 cands[i].store_mode == kStoreFused);
+    if (st != FTDX_OK && st != FTDX_ERR_ALLOC) return st;
+    if (st == FTDX_OK)
+      ++i;
+    else
+      cands.erase(cands.begin() + ptrdiff_t(i));
+  }
   st = tune_sweep(
       h, [&](const Strategy& cand, cudaStream_t ss) { return launch_all(h, c, cand, ss); },
       cands, s, &best);
@@ -646,6 +668,7 @@ ftdx_status ftdx_init_herk(ftdx_handle h, int N, int K, int batch, void* stream)
   if (!h->user_strategy && !stream_capturing(static_cast<cudaStream_t>(stream))) {
     // partial triangles for every shape up to this one; where they do not fit,
     // for this one (below)
+    h->partials.refused = 0;
     ensure_partials(h, most_split_bytes(N, K, batch), static_cast<cudaStream_t>(stream));
     return prepare_auto(h, c, static_cast<cudaStream_t>(stream), &strat);
   }

@@ -90,6 +90,16 @@ inline size_t most_split_bytes(int N, int K, int batch) {
   return sp > 1 ? std::min(kMostSplitBytes, split_bytes(N, batch, sp)) : 0;
 }
 
+// The rule's choice where have(splits) says whether the partial triangles and
+// the tile plan of that many ranges are there or can be had; else unsplit.
+template <typename Have>
+Strategy untuned_choice(int sm_count, int N, int K, int batch, bool fused_ok, bool split_ok,
+                        Have have) {
+  const Strategy s = auto_strategy(sm_count, N, K, batch, fused_ok, split_ok);
+  if (s.splits <= 1 || have(s.splits)) return s;
+  return auto_strategy(sm_count, N, K, batch, fused_ok, false);
+}
+
 // Device memory of the partial triangles, grown on demand.  A buffer that a
 // caller's graph was captured with is not freed when a larger one replaces it,
 // since every replay of that graph writes to it: it stays until release().
@@ -98,12 +108,27 @@ struct Partials {
   size_t cap = 0;
   bool captured = false;       // a caller's capture holds ptr
   std::vector<uint8_t*> held;  // replaced buffers that captures hold
+  size_t refused = 0;          // the least size that there was no memory for (0: none)
 
   // alloc(bytes) returns nullptr on failure; drop(p) waits for p's users and
-  // frees it.  False: not enough memory.
+  // frees it.  False: not enough memory, and what was there is there again.
   template <typename Alloc, typename Drop>
   bool grow(size_t bytes, Alloc alloc, Drop drop) {
     if (bytes <= cap) return true;
+    const bool ok = replace(bytes, alloc, drop);
+    if (!ok)
+      refused = refused ? std::min(refused, bytes) : bytes;
+    else if (refused && bytes >= refused)
+      refused = 0;
+    return ok;
+  }
+
+  // A size that was refused before is not asked for again until release() or
+  // until `refused` is cleared: each try would cost a failing allocation.
+  bool hopeless(size_t bytes) const { return bytes > cap && refused && bytes >= refused; }
+
+  template <typename Alloc, typename Drop>
+  bool replace(size_t bytes, Alloc alloc, Drop drop) {
     uint8_t* p = nullptr;
     if (captured) {
       // half as large again, so that all that is held stays below twice the
@@ -117,9 +142,12 @@ struct Partials {
     } else {
       if (ptr) drop(ptr);
       ptr = nullptr;
-      cap = 0;
       p = alloc(bytes);
-      if (!p) return false;
+      if (!p) {
+        if (cap) ptr = alloc(cap);
+        if (!ptr) cap = 0;
+        return false;
+      }
     }
     ptr = p;
     cap = bytes;

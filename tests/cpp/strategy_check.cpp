@@ -70,14 +70,43 @@ int partials() {
   // room for what is needed, not for half as much again
   heap.limit = heap.used + cap + 8;
   CHECK(p.grow(cap + 8, alloc, drop) && p.cap == cap + 8 && heap.live.count(last));
+  // what was refused is remembered, and more than it; less is not, nor what fits
+  heap.limit = heap.used;
+  const size_t now = p.cap;
+  CHECK(!p.grow(3 * now, alloc, drop) && p.cap == now && p.ptr);
+  const int tries = heap.allocs;
+  CHECK(p.hopeless(3 * now) && p.hopeless(4 * now) && !p.hopeless(2 * now) && !p.hopeless(now));
+  CHECK(heap.allocs == tries);
+  // a smaller one that fits does not make it forget, a larger one does
+  heap.limit = ~size_t(0);
+  CHECK(p.grow(2 * now, alloc, drop) && p.hopeless(3 * now));
+  CHECK(p.grow(3 * now, alloc, drop) && !p.hopeless(4 * now));
   p.release(drop);
   CHECK(heap.live.empty() && heap.used == 0 && !p.ptr && p.cap == 0 && p.held.empty());
+  return 0;
+}
+
+// 512 x 8192 x 4 and x 2: split by the rule, unsplit where the partials cannot be had
+int fallback() {
+  int asked = 0;
+  auto yes = [&](int sp) { return asked = sp, true; };
+  auto no = [&](int sp) { return asked = sp, false; };
+  for (int b : {4, 2})
+    for (bool fused : {false, true}) {
+      const Strategy s = untuned_choice(148, 512, 8192, b, fused, true, yes);
+      CHECK(s.splits > 1 && s.splits == asked);
+      CHECK(s == auto_strategy(148, 512, 8192, b, fused, true));
+      const Strategy u = untuned_choice(148, 512, 8192, b, fused, true, no);
+      CHECK(u == auto_strategy(148, 512, 8192, b, fused, false) && u.splits == 1);
+    }
+  asked = 0;  // nothing is asked for where the rule does not split
+  CHECK(untuned_choice(148, 2048, 1024, 16, true, true, no).splits == 1 && asked == 0);
   return 0;
 }
 }  // namespace
 
 int main() {
-  if (partials()) return 1;
+  if (partials() || fallback()) return 1;
   char cmd[16];
   while (std::scanf("%15s", cmd) == 1) {
     if (!std::strcmp(cmd, "rule")) {

@@ -126,3 +126,45 @@ def test_graph_outlives_later_calls(init):
         assert all(bool((t == 7.0).all()) for t in keep)
         assert c.device_status() == 0
         del g
+
+
+def test_no_memory_for_partials():
+    # 33.6 MB of planes fit, 12.6 MB of partial triangles do not: eager and
+    # captured calls and the tuner all go on without them
+    N, K, B = 512, 8192, 4
+    qc = oracle.gaussian_qc(31, B, N, K)
+    ref = oracle.herk_qc(qc, N, K, B).astype(np.float32)
+    d = device_bytes(qc)
+    C = torch.full((B, tri_size(N), 2), float("nan"), device=DEV)
+    s = torch.cuda.Stream()
+    with Correlator() as c:  # every kernel is loaded before the memory goes
+        c.herk(d, C, N, K, B, input=IN_INT4, output=OUT_FP32, tune=False)
+        c.tune(d, C, N, K, B)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    with Correlator() as c:
+        free = torch.cuda.mem_get_info()[0]
+        try:
+            hog = torch.empty(free - (40 << 20), dtype=torch.uint8, device=DEV)
+        except torch.cuda.OutOfMemoryError:
+            pytest.skip("device memory is in use elsewhere")
+        try:
+            c.init_herk(N, K, B)
+            c.herk(d, C, N, K, B, input=IN_INT4, output=OUT_FP32, tune=False)
+            assert np.array_equal(C.cpu().numpy(), ref)
+            C.fill_(float("nan"))
+            torch.cuda.synchronize()
+            g = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(g, stream=s):
+                c.herk(d, C, N, K, B, input=IN_INT4, output=OUT_FP32, tune=False, stream=s)
+            g.replay()
+            assert np.array_equal(C.cpu().numpy(), ref)
+            del g
+            C.fill_(float("nan"))
+            c.herk(d, C, N, K, B, input=IN_INT4, output=OUT_FP32, tune=True)
+            assert np.array_equal(C.cpu().numpy(), ref)
+            assert c.tuned_split_k(N, K, B) == 1
+            assert c.device_status() == 0
+        finally:
+            del hog
+            torch.cuda.empty_cache()
