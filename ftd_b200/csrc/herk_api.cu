@@ -190,21 +190,11 @@ ftdx_status prepare(ftdx_handle h, const HerkCall& c, cudaStream_t s, const Plan
   return get_plan(h, c.N, int(Kp / kStageK), c.batch, s, plan, pair, splits, c.out_format == 1);
 }
 
-// NVFP4: the CTA pair from four rounds of its tiles on, where the operand
-// bytes it saves per tile outweigh its coarser tiles, and from four k-blocks
-// on, where the loads and not the stores set the pace.  Single CTA / pair, us:
-// 4096 inputs x 1024 x 16: 995 / 926; 2048 x 1024 x 8 (9 rounds): 204 / 194;
-// 1500 x 1000 x 4 (3 rounds): 78 / 78; 1024 x 512 x 4: 39 / 45;
-// 4096 x 128 x 4 (one k-block): 111 / 125.
-Strategy fp4_strategy(int N, int K, int batch) {
-  const int64_t nj = (N + 255) / 256, tiles = nj * (nj + 1) * 8 / 7 * batch;  // ~ of 256 x 112
-  const int pairs = nvfp4_pair_limit();
-  return Strategy{pairs >= 1 && tiles >= 4 * pairs && nvfp4_kblocks(K) >= 4 ? 2 : 0, 0};
-}
-
 Strategy untuned_strategy(ftdx_handle h, const HerkCall& c) {
   if (h->user_strategy) return h->default_strategy;
-  if (is_fp4(c)) return fp4_strategy(c.N, c.K, c.batch);
+  if (is_fp4(c))
+    return fp4_strategy(nvfp4_pair_limit(), c.N, nvfp4_kblocks(c.K), c.batch,
+                        c.compute == FTDX_COMPUTE_FP4_SPLIT);
   return auto_strategy(h->sm_count, c.N, c.K, c.batch, fused_ok(c), !c.comp && c.out_format == 0);
 }
 

@@ -80,6 +80,27 @@ inline Strategy auto_strategy(int sm_count, int N, int K, int batch, bool fused_
   return best;
 }
 
+// NVFP4 without a strategy of the user's: the CTA pair where the operand bytes
+// it saves per k-block outweigh its coarser tiles -- more than four blocks of 256
+// inputs, four rounds of its tiles, four k-blocks (of 128 samples), and 40
+// products of k-blocks per pair (hi + lo has three per k-block).  Single CTA /
+// pair, us, 74 pairs, Gaussian voltages:
+//   plain   2048 x 1024 x 8 (9 rounds of 8): 169 / 158; 4096 x 1024 x 2: 129 / 113;
+//           1500 x 700 x 14 (9 of 6): 144 / 137; 1700 x 700 x 6 (5 of 6): 77 / 80;
+//           2048 x 512 x 5 (5 of 4): 60 / 66; 4096 x 512 x 1 (4 of 4): 43 / 45;
+//           2048 x 300 x 14 (16 of 3): 144 / 151;
+//   hi + lo 2048 x 512 x 4 (4 of 4): 89 / 83; 1100 x 1024 x 19: 286 / 265;
+//   up to 1024 inputs, both: 1024 x 512 x 16: 74 / 80 and 115 / 125; 512 x 1024
+//           x 65: 204 / 206 and 311 / 327; 300 x 1024 x 97: 164 / 177 and 245 / 272.
+// Of 374 shapes of 300 to 4096 inputs, both modes, none that takes the pair is
+// more than 4% behind the single CTA.
+inline Strategy fp4_strategy(int pairs, int N, int kblocks, int batch, bool split) {
+  const int64_t nj = (N + 255) / 256, tiles = nj * (nj + 1) * 8 / 7 * batch;  // ~ of 256 x 112
+  const int64_t work = tiles * kblocks * (split ? 3 : 1);
+  const bool pair = pairs >= 1 && nj > 4 && tiles >= 4 * pairs && kblocks >= 4 && work >= 40 * pairs;
+  return Strategy{pair ? 2 : 0, 0};
+}
+
 // The most bytes of partial triangles that auto_strategy takes for any shape up
 // to (N, K, batch).  A smaller shape can take more than a larger one: on 148 SMs
 // 512 inputs x 8192 samples take three ranges for 4 channels (12.6 MB) and seven

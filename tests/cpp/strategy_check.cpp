@@ -1,7 +1,8 @@
 // Host checks of strategy.h: the untuned rule over commands on standard input,
 // and the growth of the split-K partial buffer with an allocator that counts
 // and can fail.  "rule SMS N K BATCH FUSED SPLIT" answers "MODE SPLITS BYTES",
-// "bound N K BATCH" the bytes that cover every shape up to that one.
+// "bound N K BATCH" the bytes that cover every shape up to that one, "fp4 PAIRS N
+// KBLOCKS BATCH SPLIT" the NVFP4 kernel's store mode.
 #include <cstdio>
 #include <cstring>
 #include <map>
@@ -119,6 +120,10 @@ int main() {
       int n, k, b;
       if (std::scanf("%d %d %d", &n, &k, &b) != 3) return 2;
       std::printf("%zu\n", most_split_bytes(n, k, b));
+    } else if (!std::strcmp(cmd, "fp4")) {
+      int pairs, n, kb, b, s;
+      if (std::scanf("%d %d %d %d %d", &pairs, &n, &kb, &b, &s) != 5) return 2;
+      std::printf("%d\n", fp4_strategy(pairs, n, kb, b, s != 0).store_mode);
     }
   }
   return 0;

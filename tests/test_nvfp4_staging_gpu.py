@@ -35,8 +35,8 @@ def test_matches_restated_quantiser(K, offset):
             assert err[:, ~diag].max() <= tol * np.abs(ref).max()
 
 
-# a size that takes the pair, and the same shape with too short a K for it
-@pytest.mark.parametrize("N,K,B", [(2048, 512, 4), (2048, 128, 4)])
+# a size that takes the pair, and shapes with too few k-blocks or rounds for it
+@pytest.mark.parametrize("N,K,B", [(2048, 1024, 8), (2048, 512, 4), (2048, 128, 4)])
 def test_untuned_equals_both_kernels(N, K, B):
     g = torch.Generator(device=DEV).manual_seed(5)
     A = torch.randn(B, N, K, 2, device=DEV, generator=g)

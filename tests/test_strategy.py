@@ -50,3 +50,15 @@ def test_bound_covers_every_smaller_shape(check):
         split += sum(c > 0 for c in caps)
         assert max(caps) <= out[i][0]
     assert split > 500
+
+
+# pairs, inputs, k-blocks, channels, hi + lo: what was measured slower on the CTA
+# pair stays on the single CTA, what was faster takes the pair
+@pytest.mark.parametrize("args,mode", [
+    ((74, 1024, 4, 16, 0), 0), ((74, 1024, 4, 16, 1), 0), ((74, 1024, 16, 52, 1), 0),
+    ((74, 512, 8, 65, 1), 0), ((74, 300, 8, 97, 0), 0), ((74, 2048, 4, 5, 0), 0),
+    ((74, 2048, 3, 14, 0), 0), ((74, 1500, 16, 3, 1), 0), ((0, 4096, 8, 16, 0), 0),
+    ((74, 1100, 8, 19, 1), 2), ((74, 2048, 4, 4, 1), 2), ((74, 2048, 8, 8, 0), 2),
+    ((74, 4096, 8, 16, 0), 2), ((74, 4096, 4, 4, 0), 2)])
+def test_nvfp4_kernel(check, args, mode):
+    assert check(["fp4 " + " ".join(str(a) for a in args)]) == [(mode,)]
