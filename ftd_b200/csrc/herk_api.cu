@@ -673,6 +673,7 @@ ftdx_status ftdx_end_herk(ftdx_handle h) {
   if (h->z) cudaFree(h->z);
   h->z = nullptr;
   h->z_cap = 0;
+  h->partials.release([](uint8_t* p) { cudaFree(p); });
   h->plans.clear();
   h->vplans.clear();
   return FTDX_OK;

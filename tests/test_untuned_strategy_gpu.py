@@ -168,3 +168,22 @@ def test_no_memory_for_partials():
         finally:
             del hog
             torch.cuda.empty_cache()
+
+
+def test_end_herk_gives_the_partials_back():
+    N, K, B = 512, 8192, 4
+    qc = oracle.gaussian_qc(41, B, N, K)
+    d = device_bytes(qc)
+    C = torch.full((B, tri_size(N), 2), float("nan"), device=DEV)
+    with Correlator() as c:
+        c.herk(d, C, N, K, B, input=IN_INT4, output=OUT_FP32, tune=False)  # kernels loaded
+        c.end_herk()
+        free = torch.cuda.mem_get_info()[0]
+        c.init_herk(N, K, B)
+        assert torch.cuda.mem_get_info()[0] <= free - (100 << 20)  # planes and partials
+        c.herk(d, C, N, K, B, input=IN_INT4, output=OUT_FP32, tune=False)
+        c.end_herk()
+        assert torch.cuda.mem_get_info()[0] >= free
+        c.herk(d, C, N, K, B, input=IN_INT4, output=OUT_FP32, tune=False)
+        assert c.device_status() == 0
+    assert np.array_equal(C.cpu().numpy(), oracle.herk_qc(qc, N, K, B).astype(np.float32))
