@@ -85,7 +85,8 @@ struct ftdx_context {
   std::map<std::tuple<int, int, int>, std::unique_ptr<ftdx::Plan>> plans;  // (N, kblocks, batch)
   std::map<uint64_t, std::shared_ptr<void>> vplans;  // batched-call plans by fingerprint
   // strategy of untuned calls once the user has set one (ftdx_set_strategy,
-  // ftdx_set_split_k); until then the call's sizes decide
+  // ftdx_set_split_k); until then, and after ftdx_clear_strategy, the call's
+  // sizes decide
   ftdx::Strategy default_strategy;
   bool user_strategy = false;
   // autotuner
@@ -150,8 +151,6 @@ struct ScopedTimer {
 };
 
 void release_graphs(ftdx_handle h);
-// Back to no strategy of the user's (a new handle's state).
-void clear_strategy(ftdx_handle h);
 void load_tune_cache(ftdx_handle h);
 
 // Autotuning and graph replay shared by the correlator entry points.

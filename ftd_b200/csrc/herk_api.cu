@@ -431,11 +431,6 @@ ftdx_status run_graph(ftdx_handle h, const HerkCall& c, const Strategy& strat, c
 
 }  // namespace
 
-void clear_strategy(ftdx_handle h) {
-  h->default_strategy = Strategy{};
-  h->user_strategy = false;
-}
-
 std::vector<Strategy> default_candidates(ftdx_handle h, bool fp32_out, bool pair_ok) {
   std::vector<Strategy> v;
   const int grids[2] = {h->sm_count, h->sm_count - h->sm_count / 8};
@@ -898,6 +893,13 @@ ftdx_status ftdx_set_strategy(ftdx_handle h, int store_mode, int grid) {
   }
   h->default_strategy = Strategy{store_mode, grid, h->default_strategy.splits};
   h->user_strategy = true;
+  return FTDX_OK;
+}
+
+ftdx_status ftdx_clear_strategy(ftdx_handle h) {
+  if (!h) return FTDX_ERR_INVALID_ARG;
+  h->default_strategy = Strategy{};
+  h->user_strategy = false;
   return FTDX_OK;
 }
 

@@ -8,10 +8,6 @@
 
 #include "ftdx.h"
 
-namespace ftdx {
-void clear_strategy(ftdx_handle h);  // herk_api.cu
-}
-
 namespace cutlass_gemm_api {
 
 struct CutlassComplexGemm::Impl {
@@ -52,7 +48,7 @@ struct CutlassComplexGemm::Impl {
         if (ftdx_set_strategy(h, 2, 0) != FTDX_OK) ftdx_set_strategy(h, 0, 0);
         break;
       case HerkMode::ForceDirect: ftdx_set_strategy(h, 0, 0); break;
-      case HerkMode::Auto: ftdx::clear_strategy(h); break;
+      case HerkMode::Auto: ftdx_clear_strategy(h); break;
     }
   }
 };

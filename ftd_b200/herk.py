@@ -257,6 +257,10 @@ class Correlator:
         if splits is not None:
             check(self._h, self._L.ftdx_set_split_k(self._h, splits), "ftdx_set_split_k")
 
+    def clear_strategy(self) -> None:
+        """Let the call's sizes decide again, as on a new handle (ftdx_clear_strategy)."""
+        check(self._h, self._L.ftdx_clear_strategy(self._h), "ftdx_clear_strategy")
+
     def tuned_split_k(self, N: int, K: int, batch: int, input: int = IN_INT4,
                       output: int = OUT_FP32) -> int:
         """Split-K count the autotuner recorded for this shape (-1: none)."""

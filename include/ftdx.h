@@ -290,7 +290,11 @@ FTDX_API ftdx_status ftdx_herk_kahan(ftdx_handle h, const void* A, void* sum, vo
                                      void* stream);
 
 /* Pre-size the workspace for problems up to (N, K, batch) so that later
- * ftdx_herk calls allocate nothing (required before graph capture).
+ * ftdx_herk calls allocate nothing (required before graph capture).  On a
+ * handle without a strategy that includes split-K partial triangles for any
+ * shape up to this one, at most 256 MB; where they do not fit, calls run
+ * unsplit.  ftdx_end_herk frees all of it (after it, graphs that the caller
+ * captured from this handle must not be replayed).
  * Replaces CutlassComplexGemm::init_herk / end_herk (cutlass_gemm_api.h:617-624). */
 FTDX_API ftdx_status ftdx_init_herk(ftdx_handle h, int N, int K, int batch, void* stream);
 FTDX_API ftdx_status ftdx_end_herk(ftdx_handle h);
@@ -339,10 +343,15 @@ FTDX_API ftdx_status ftdx_set_graph_mode(ftdx_handle h, int enable);
 FTDX_API int ftdx_graph_count(ftdx_handle h);
 
 /* Strategy for calls that are not tuned (tune = 0, or no cache entry).  Until
- * this or ftdx_set_split_k is called on a handle, the library picks by the
- * call's sizes: the single-CTA kernel with direct stores, INT4 promotion
- * apart or fused in (modes 0 and 16), and split-K where the tiles leave SMs
- * idle.
+ * this or ftdx_set_split_k is called on a handle, and after
+ * ftdx_clear_strategy, the library picks by the call's sizes: the single-CTA
+ * kernel with direct stores, INT4 promotion apart or fused in (modes 0 and 16),
+ * and split-K where the tiles leave SMs idle; for NVFP4 the single CTA or the
+ * pair.  The split count follows the number of channels (and of SMs), so the
+ * FP32 order of sums of a channel of FP16 or FP32 input does too: the same
+ * channel in a call of another batch may differ in the last bits.  INT4 results
+ * below 2^24 are exact integers whatever the split.  ftdx_set_strategy(h, 0, 0)
+ * gives the same bits at any batch.
  * store_mode 0 = direct stores, 1 = shared-memory staging + bulk copies,
  * 2 = CTA-pair kernel (one tcgen05 cta_group::2 MMA over two SMs per
  * 256 x 128 tile; uniform ftdx_herk calls, ftdx_herk_batched_v and
@@ -366,6 +375,10 @@ FTDX_API int ftdx_graph_count(ftdx_handle h);
  * store_mode 2, 3, 2 + 8, 3 + 8 and 16 for uniform INT4 calls, 2 and 3 for
  * ftdx_herk_batched_v, and both NVFP4 kernels. */
 FTDX_API ftdx_status ftdx_set_strategy(ftdx_handle h, int store_mode, int grid);
+
+/* Back to a new handle's state: the call's sizes decide again (strategy and
+ * split count). */
+FTDX_API ftdx_status ftdx_clear_strategy(ftdx_handle h);
 
 /* Split-K for untuned calls: K is cut into `splits` (1..32) ranges of
  * k-blocks, each correlated into its own partial triangle, and a reduction

@@ -51,6 +51,7 @@ def test_null_arguments_rejected_without_gpu():
     L = _lib.load()
     assert L.ftdx_create(None, None) == 1
     assert L.ftdx_destroy(None) == 1
+    assert L.ftdx_clear_strategy(None) == 1
     assert L.ftdx_herk(None, None, None, 1, 1, 1, 1, 0, 1, 0, 1.0, 0.0, None, 0) == 1
 
 
