@@ -42,3 +42,30 @@ def test_first_rows_match_the_restated_quantiser(N, K, B):
             for b in range(B):
                 assert np.abs(got[b] - ref[b]).max() <= tol * np.abs(ref[b]).max()
             assert bool(torch.isfinite(C).all())
+
+
+# more channels than a grid has rows, on the path of short channels
+@pytest.mark.parametrize("compute,split", [(COMPUTE_FP8, False), (COMPUTE_FP8_SPLIT, True)])
+def test_more_than_65535_channels(compute, split):
+    N, K, B = 2, 16, 65537
+    g = torch.Generator(device=DEV).manual_seed(7)
+    A = torch.randn(B, N, K, 2, device=DEV, generator=g)
+    A *= torch.exp(4 * torch.randn(B, 1, 1, 1, device=DEV, generator=g))
+    C = torch.full((B, tri_size(N), 2), float("nan"), device=DEV)
+    with Correlator() as c:
+        c.herk(A, C, N, K, B, input=IN_FP32, compute=compute, output=OUT_FP32, tune=False)
+        assert c.device_status() == 0
+    got = C.double().cpu().numpy()
+    v = np.ascontiguousarray(A.cpu().numpy()).view(np.complex64)[..., 0]
+    for b in (0, 1, 65534, 65535, 65536):
+        tol = (3 if split else 1) * (K / 16 + 2) * 2.0 ** -24  # as above
+        ref = oracle.herk_fp8_scaled(v[b:b + 1], split)[0]
+        assert np.abs(got[b] - ref).max() <= tol * np.abs(ref).max()
+    # every channel: E4M3 rounds each part by at most 2^-4 of it, so a product of
+    # two by 2^-3 + 2^-8, and what is below its normal range by 2^-10 of 1 / scale
+    w = v.astype(np.complex128)
+    i, j = np.array([0, 1, 1]), np.array([0, 0, 1])
+    bound = 0.13 * (np.abs(w[:, i]) * np.abs(w[:, j])).sum(-1)
+    bound += 1e-4 * np.abs(w).max(axis=(1, 2))[:, None] ** 2
+    exact = (w[:, i] * np.conj(w[:, j])).sum(-1)
+    assert (np.abs(got[..., 0] + 1j * got[..., 1] - exact) <= bound).all()
