@@ -313,7 +313,7 @@ __global__ void __launch_bounds__(256) nvfp4_stats_kernel(
 // carry a lo residual.  src[p] = the source sample of position p (-1:
 // padding); nflag[c] = F; chans[c].pad = number of trailing k-blocks (of
 // 128 samples) with a lo residual (all of them in split mode).
-__global__ void __launch_bounds__(1024) nvfp4_order_kernel(const uint32_t* __restrict__ flags,
+__global__ void __launch_bounds__(1024) nvfp4_order_kernel(const uint32_t* flags,
                                                            int32_t* __restrict__ src,
                                                            int32_t* __restrict__ nflag,
                                                            ChanDesc* __restrict__ chans, int K,
@@ -383,9 +383,8 @@ constexpr int kStageSamples = 1024;
 __host__ __device__ constexpr size_t stage_bytes_per_row(int K) { return size_t((K + 7) / 8) * 9 * sizeof(float2); }
 template <bool kStaged>
 __global__ void __launch_bounds__(256, kStaged ? 3 : 4) nvfp4_quant_kernel(
-    const float2* __restrict__ a, const int32_t* __restrict__ src,
-    const int32_t* __restrict__ nflag, const ChanDesc* __restrict__ chans,
-    const float* __restrict__ rscale, uint8_t* __restrict__ z, uint8_t* __restrict__ sfa,
+    const float2* __restrict__ a, const int32_t* src, const int32_t* nflag,
+    const ChanDesc* chans, const float* rscale, uint8_t* __restrict__ z, uint8_t* __restrict__ sfa,
     uint8_t* __restrict__ sfb, int64_t rows, int K, int kp, int pitch, SfGeom sg) {
   griddep_wait();  // row scales and time order
   griddep_launch();
@@ -396,9 +395,9 @@ __global__ void __launch_bounds__(256, kStaged ? 3 : 4) nvfp4_quant_kernel(
   for (int64_t r = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; r < rows;
        r += (int64_t(gridDim.x) * blockDim.x) >> 5) {
     const float2* p = a + r * K;
-    const float g = __ldg(rscale + r);
+    const float g = rscale[r];
     const int c = int(r / sg.n), w = int(r - int64_t(c) * sg.n);
-    const bool permuted = __ldg(nflag + c) > 0;
+    const bool permuted = nflag[c] > 0;
     const int lo_from = (kp / 128 - chans[c].pad) * 16;  // first block with a residual
     const int32_t* sc = src + int64_t(c) * kp;
     const Fp4RowOut o = fp4_row_out(r, c, w, z, sfa, sfb, pitch, sg);
@@ -439,8 +438,8 @@ __global__ void __launch_bounds__(256, kStaged ? 3 : 4) nvfp4_quant_kernel(
           // positions past K have source -1 (t0 < kp: the order covers the padding)
           int src8[8];
           if (permuted) {
-            const int4 s0 = __ldg(reinterpret_cast<const int4*>(sc + t0));
-            const int4 s1 = __ldg(reinterpret_cast<const int4*>(sc + t0) + 1);
+            const int4 s0 = *reinterpret_cast<const int4*>(sc + t0);
+            const int4 s1 = *(reinterpret_cast<const int4*>(sc + t0) + 1);
             src8[0] = s0.x, src8[1] = s0.y, src8[2] = s0.z, src8[3] = s0.w;
             src8[4] = s1.x, src8[5] = s1.y, src8[6] = s1.z, src8[7] = s1.w;
           } else {
@@ -470,7 +469,7 @@ __global__ void __launch_bounds__(256, kStaged ? 3 : 4) nvfp4_quant_kernel(
         } else {
 #pragma unroll
           for (int q = 0; q < 8; ++q) {
-            const int t = permuted ? (t0 + q < kp ? __ldg(sc + t0 + q) : -1) : (t0 + q < K ? t0 + q : -1);
+            const int t = permuted ? (t0 + q < kp ? sc[t0 + q] : -1) : (t0 + q < K ? t0 + q : -1);
             const float2 v = t >= 0 ? __ldg(p + t) : make_float2(0.f, 0.f);
             x[2 * q] = v.x, x[2 * q + 1] = v.y;
           }

@@ -1359,11 +1359,11 @@ cudaError_t launch_herk_fp8_pair(const CUtensorMap& tmZ, const HerkArgs& a, int 
 // (ws[c*splits + s][P]); C = alpha * cs_c * sum_s partial_s + beta * C.  The
 // partials of integer inputs are exact integers, so the sum is too.
 template <typename Out2>
-__global__ void __launch_bounds__(256) split_reduce_kernel(const float2* __restrict__ ws,
+__global__ void __launch_bounds__(256) split_reduce_kernel(const float2* ws,
                                                            Out2* __restrict__ out, int64_t P,
                                                            int batch, int splits, float alpha,
                                                            float beta,
-                                                           const float* __restrict__ chan_scale) {
+                                                           const float* chan_scale) {
   griddep_wait();
   const int64_t total = int64_t(batch) * P;
   for (int64_t x = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; x < total;

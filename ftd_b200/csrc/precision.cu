@@ -164,7 +164,7 @@ __device__ __forceinline__ void span_e4m3(const float (&xr)[8], const float (&xi
 __global__ void __launch_bounds__(256) quantize_kernel(const float2* __restrict__ a,
                                                        uint8_t* __restrict__ z, int64_t rows,
                                                        int K, int Kp, int zpitch, int n,
-                                                       const uint32_t* __restrict__ amax_bits,
+                                                       const uint32_t* amax_bits,
                                                        float* __restrict__ out_scale, int split,
                                                        int rows_per_block, int vec) {
   __shared__ __align__(16) uint32_t bytes[16][64];
@@ -186,7 +186,7 @@ __global__ void __launch_bounds__(256) quantize_kernel(const float2* __restrict_
     const int64_t r = r0 + rl;
     const int c = c0 + (rin0 + rl) / n;
     if (c != cs) {
-      s = channel_scale(__uint_as_float(__ldg(amax_bits + c)));
+      s = channel_scale(__uint_as_float(amax_bits[c]));
       cs = c;
     }
     if (t0 == 0 && r == int64_t(c) * n) out_scale[c] = 1.f / (s * s);
