@@ -50,7 +50,9 @@ def _stream(s) -> int:
     never imported is not looked for and no Stream object is made."""
     if s is None:
         torch = sys.modules.get("torch")
-        if torch is None or not torch.cuda.is_initialized():
+        # no torch, or one that another thread is still importing: no CUDA work of its
+        ready = getattr(getattr(torch, "cuda", None), "is_initialized", None)
+        if ready is None or not ready():
             return 0
         raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
         if raw is not None:
