@@ -107,6 +107,7 @@ PROTOTYPES = {
     "ftdx_graph_count": (_i, [_vp]),
     "ftdx_set_strategy": (_i, [_vp, _i, _i]),
     "ftdx_clear_strategy": (_i, [_vp]),
+    "ftdx_last_strategy": (_i, [_vp, ctypes.POINTER(_i), ctypes.POINTER(_i), ctypes.POINTER(_i)]),
     "ftdx_set_split_k": (_i, [_vp, _i]),
     "ftdx_tuned_split_k": (_i, [_vp, _i, _i, _i, _i, _i]),
     "ftdx_herk_static": (_i, [_vp, _vp, _i, _i, _i, _vp, ctypes.POINTER(ctypes.c_uint32),

@@ -89,6 +89,7 @@ struct ftdx_context {
   // sizes decide
   ftdx::Strategy default_strategy;
   bool user_strategy = false;
+  ftdx::Strategy last;  // what the last correlator call launched (ftdx_last_strategy)
   // autotuner
   std::string tune_cache;
   std::map<ftdx::TuneKey, ftdx::TuneEntry> tuned;

@@ -123,6 +123,7 @@ ftdx_status launch_fp4(ftdx_handle h, const HerkCall& c, const Strategy& strat, 
   const int64_t rows = int64_t(c.N) * c.batch;
   const int split = c.compute == FTDX_COMPUTE_FP4_SPLIT ? 1 : 0;
   const int pair = ((strat.store_mode & 3) >= 2 && nvfp4_pair_limit() >= 1) ? 1 : 0;
+  h->last = Strategy{pair ? 2 : 0, 0};
   ftdx_status st = ensure_workspace(h, nvfp4_workspace_bytes(c.N, c.batch, c.K, split, pair), s);
   const Plan* plan = nullptr;
   if (st == FTDX_OK)
@@ -236,6 +237,8 @@ ftdx_status launch_all(ftdx_handle h, const HerkCall& c, const Strategy& strat, 
   const bool pair = use_pair(h, strat);
   const bool fused = strat.store_mode == kStoreFused && fused_ok(c);
   const int splits = effective_splits(c, strat);
+  h->last = Strategy{strat.store_mode == kStoreFused && !fused ? 0 : strat.store_mode, strat.grid,
+                     splits};
   const Plan* plan = nullptr;
   ftdx_status st = prepare(h, c, s, &plan, pair, splits, fused);
   if (st != FTDX_OK) return st;
@@ -900,6 +903,14 @@ ftdx_status ftdx_clear_strategy(ftdx_handle h) {
   if (!h) return FTDX_ERR_INVALID_ARG;
   h->default_strategy = Strategy{};
   h->user_strategy = false;
+  return FTDX_OK;
+}
+
+ftdx_status ftdx_last_strategy(ftdx_handle h, int* store_mode, int* grid, int* splits) {
+  if (!h) return FTDX_ERR_INVALID_ARG;
+  if (store_mode) *store_mode = h->last.store_mode;
+  if (grid) *grid = h->last.grid;
+  if (splits) *splits = h->last.splits;
   return FTDX_OK;
 }
 

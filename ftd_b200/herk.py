@@ -263,6 +263,13 @@ class Correlator:
         """Let the call's sizes decide again, as on a new handle (ftdx_clear_strategy)."""
         check(self._h, self._L.ftdx_clear_strategy(self._h), "ftdx_clear_strategy")
 
+    def last_strategy(self) -> dict:
+        """What the last correlator call launched (ftdx_last_strategy)."""
+        sm, g, sp = ctypes.c_int(0), ctypes.c_int(0), ctypes.c_int(0)
+        check(self._h, self._L.ftdx_last_strategy(self._h, ctypes.byref(sm), ctypes.byref(g),
+                                                  ctypes.byref(sp)), "ftdx_last_strategy")
+        return {"store_mode": sm.value, "grid": g.value, "splits": sp.value}
+
     def tuned_split_k(self, N: int, K: int, batch: int, input: int = IN_INT4,
                       output: int = OUT_FP32) -> int:
         """Split-K count the autotuner recorded for this shape (-1: none)."""

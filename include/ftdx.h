@@ -380,6 +380,11 @@ FTDX_API ftdx_status ftdx_set_strategy(ftdx_handle h, int store_mode, int grid);
  * split count). */
 FTDX_API ftdx_status ftdx_clear_strategy(ftdx_handle h);
 
+/* The strategy that the last correlator call on this handle launched, however
+ * it was chosen (ftdx_herk, _ftd, _kahan and ftdx_xengine; a replay by graph
+ * mode does not change it). */
+FTDX_API ftdx_status ftdx_last_strategy(ftdx_handle h, int* store_mode, int* grid, int* splits);
+
 /* Split-K for untuned calls: K is cut into `splits` (1..32) ranges of
  * k-blocks, each correlated into its own partial triangle, and a reduction
  * pass adds them (C = alpha * sum + beta * C).  Fills the GPU when a call has

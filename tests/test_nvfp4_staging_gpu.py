@@ -35,9 +35,10 @@ def test_matches_restated_quantiser(K, offset):
             assert err[:, ~diag].max() <= tol * np.abs(ref).max()
 
 
-# a size that takes the pair, and shapes with too few k-blocks or rounds for it
-@pytest.mark.parametrize("N,K,B", [(2048, 1024, 8), (2048, 512, 4), (2048, 128, 4)])
-def test_untuned_equals_both_kernels(N, K, B):
+# a size that takes the pair, and shapes with too few k-blocks, rounds or inputs for it
+@pytest.mark.parametrize("N,K,B,pair", [(2048, 1024, 8, 2), (2048, 512, 4, 0), (2048, 128, 4, 0),
+                                        (1024, 512, 16, 0)])
+def test_untuned_equals_both_kernels(N, K, B, pair):
     g = torch.Generator(device=DEV).manual_seed(5)
     A = torch.randn(B, N, K, 2, device=DEV, generator=g)
     outs = []
@@ -47,6 +48,7 @@ def test_untuned_equals_both_kernels(N, K, B):
             if mode is not None:
                 c.set_strategy(mode, 0)
             c.herk(A, C, N, K, B, input=IN_FP32, compute=COMPUTE_FP4, output=OUT_FP32, tune=False)
+            assert c.last_strategy()["store_mode"] == (pair if mode is None else mode)
             assert c.device_status() == 0
         outs.append(C)
     scale = float(outs[0].abs().max())
