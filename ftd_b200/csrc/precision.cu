@@ -34,46 +34,43 @@ namespace {
 // two samples (16 bytes) per load, four loads in flight; `vec` (uniform)
 // says the channel starts 16-byte aligned and per_chan is even.
 __global__ void __launch_bounds__(256) amax_kernel(const float2* __restrict__ a, int64_t per_chan,
-                                                   int batch, uint32_t* __restrict__ amax_bits,
-                                                   int vec) {
+                                                   uint32_t* __restrict__ amax_bits, int vec) {
   dev::griddep_launch();
-  __shared__ float wm[8];
+  const int c = blockIdx.y;
+  const float2* p = a + int64_t(c) * per_chan;
+  float m = 0.f;
   const int64_t stride = int64_t(gridDim.x) * blockDim.x;
   const int64_t t0 = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  for (int c = blockIdx.y; c < batch; c += gridDim.y) {
-    const float2* p = a + int64_t(c) * per_chan;
-    float m = 0.f;
-    if (vec) {
-      const float4* p4 = reinterpret_cast<const float4*>(p);
-      const int64_t n4 = per_chan >> 1;
-      int64_t i = t0;
-      for (; i + 3 * stride < n4; i += 4 * stride) {
-        float4 v[4];
+  if (vec) {
+    const float4* p4 = reinterpret_cast<const float4*>(p);
+    const int64_t n4 = per_chan >> 1;
+    int64_t i = t0;
+    for (; i + 3 * stride < n4; i += 4 * stride) {
+      float4 v[4];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) v[u] = __ldg(p4 + i + u * stride);
+      for (int u = 0; u < 4; ++u) v[u] = __ldg(p4 + i + u * stride);
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
-          m = fmaxf(m, fmaxf(fmaxf(fabsf(v[u].x), fabsf(v[u].y)), fmaxf(fabsf(v[u].z), fabsf(v[u].w))));
-      }
-      for (; i < n4; i += stride) {
-        const float4 v = __ldg(p4 + i);
-        m = fmaxf(m, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
-      }
-    } else {
-      for (int64_t i = t0; i < per_chan; i += stride) {
-        const float2 v = __ldg(p + i);
-        m = fmaxf(m, fmaxf(fabsf(v.x), fabsf(v.y)));
-      }
+      for (int u = 0; u < 4; ++u)
+        m = fmaxf(m, fmaxf(fmaxf(fabsf(v[u].x), fabsf(v[u].y)), fmaxf(fabsf(v[u].z), fabsf(v[u].w))));
     }
-    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if ((threadIdx.x & 31) == 0) wm[threadIdx.x >> 5] = m;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      for (int w = 1; w < int(blockDim.x >> 5); ++w) m = fmaxf(m, wm[w]);
-      if (!(m == m)) m = 0.f;  // NaN input: treat as empty
-      atomicMax(amax_bits + c, __float_as_uint(m));
+    for (; i < n4; i += stride) {
+      const float4 v = __ldg(p4 + i);
+      m = fmaxf(m, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
     }
-    __syncthreads();  // wm has been read
+  } else {
+    for (int64_t i = t0; i < per_chan; i += stride) {
+      const float2 v = __ldg(p + i);
+      m = fmaxf(m, fmaxf(fabsf(v.x), fabsf(v.y)));
+    }
+  }
+  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+  __shared__ float wm[8];
+  if ((threadIdx.x & 31) == 0) wm[threadIdx.x >> 5] = m;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < int(blockDim.x >> 5); ++w) m = fmaxf(m, wm[w]);
+    if (!(m == m)) m = 0.f;  // NaN input: treat as empty
+    atomicMax(amax_bits + c, __float_as_uint(m));
   }
 }
 
@@ -441,9 +438,12 @@ cudaError_t launch_channel_amax(const void* a, int64_t per_chan, int batch, uint
   if (bx > cap) bx = cap;
   if (bx < 1) bx = 1;
   const int vec = (per_chan % 2 == 0) && (reinterpret_cast<uintptr_t>(a) & 15) == 0;
-  const int by = batch < 65535 ? batch : 65535;  // the limit of a grid's y
-  amax_kernel<<<dim3(unsigned(bx), unsigned(by)), 256, 0, s>>>(static_cast<const float2*>(a),
-                                                                per_chan, batch, amax_bits, vec);
+  // one grid row per channel, as many launches as that takes (blocks that step
+  // through the channels lose 7%: 83 against 77 us for 16 channels of 33.6 MB)
+  constexpr int kMostRows = 65535;
+  for (int c = 0; c < batch; c += kMostRows)
+    amax_kernel<<<dim3(unsigned(bx), unsigned(std::min(batch - c, kMostRows))), 256, 0, s>>>(
+        static_cast<const float2*>(a) + int64_t(c) * per_chan, per_chan, amax_bits + c, vec);
   return cudaGetLastError();
 }
 
