@@ -1239,21 +1239,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kHerkThreads, 1)
 }
 
 // ------------------------------------------------------------------ launchers
-// Rows per block of a promotion pass over `rows` rows of `chunks` per-thread
-// pieces: about eight blocks of 256 threads for each of 148 SMs while the
-// problem has that many, at most 32 pieces per thread (rows stay together, and
-// fewer blocks start) and at least one.  One fixed size of 8192 pieces gave
-// 32 channels of 128 x 256 eight blocks (21.9 us of promotion) and 16 of
-// 1024 x 1024 FP16 samples 256 (24.6 us).
-int promotion_rows_per_block(int64_t rows, int chunks) {
-  constexpr int64_t kBlocks = 8 * 148;
-  const int64_t most = 8192 / chunks, least = (256 + chunks - 1) / chunks;
-  int64_t r = rows / kBlocks;
-  if (r < least) r = least;
-  if (r > most) r = most;
-  return r < 1 ? 1 : int(r);
-}
-
 cudaError_t launch_qc_to_planes(const uint8_t* qc, uint8_t* z, int64_t rows, int K, int Kp,
                                 cudaStream_t s, bool neg_plane) {
   const int rpb = promotion_rows_per_block(rows, Kp >> 4);

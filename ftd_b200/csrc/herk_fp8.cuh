@@ -180,9 +180,6 @@ cudaError_t ensure_smem_limit(const void* kernel, size_t bytes);
 // the calling thread; ftdx_last_error(NULL) returns it (ftdx_api.cu).
 void set_thread_error(const char* fmt, ...);
 
-// Rows per block of a promotion pass over `rows` rows of `chunks` per-thread
-// pieces (herk_fp8.cu).
-int promotion_rows_per_block(int64_t rows, int chunks);
 // Launches `kernel`, which calls griddep_wait() before it touches anything that
 // the kernel queued before it writes: its start (barriers, TMEM, descriptor
 // prefetch) then overlaps that kernel's end.  Without such a kernel in front, or

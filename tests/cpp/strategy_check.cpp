@@ -104,10 +104,23 @@ int fallback() {
   CHECK(untuned_choice(148, 2048, 1024, 16, true, true, no).splits == 1 && asked == 0);
   return 0;
 }
+
+// a promotion's blocks are all resident at once unless 32 pieces per thread are not enough
+int promotion() {
+  for (int chunks : {8, 16, 24, 64, 128, 250, 256, 512, 8192, 10000})
+    for (int64_t rows = 1; rows < 3000000; rows += 1 + rows / 7) {
+      const int64_t r = promotion_rows_per_block(rows, chunks), blocks = (rows + r - 1) / r;
+      CHECK(r >= 1 && (r == 1 || r * chunks <= 8192));
+      CHECK(blocks <= kPromotionBlocks || (r + 1) * chunks > 8192);
+      CHECK(r * chunks >= 256 || chunks > 8192);
+      CHECK((r - 1) * chunks < 256 || (rows + r - 2) / (r - 1) > kPromotionBlocks);  // no larger than it must
+    }
+  return 0;
+}
 }  // namespace
 
 int main() {
-  if (partials() || fallback()) return 1;
+  if (partials() || fallback() || promotion()) return 1;
   char cmd[16];
   while (std::scanf("%15s", cmd) == 1) {
     if (!std::strcmp(cmd, "rule")) {

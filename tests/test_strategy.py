@@ -1,7 +1,7 @@
 """The untuned rule and the split-K partial buffer, on the CPU: the buffer that
 a caller's graph was captured with outlives its replacement, a failed allocation
-leaves the unsplit kernel, and init_herk's size covers every shape up to the one
-it was given."""
+leaves the unsplit kernel, init_herk's size covers every shape up to the one it was
+given, and the blocks of a promotion pass are resident at once."""
 import os
 import random
 import subprocess
@@ -25,7 +25,7 @@ def check(tmp_path_factory):
     return run
 
 
-def test_partial_buffer_and_fallback(check):
+def test_partial_buffer_fallback_and_promotion_blocks(check):
     assert check([]) == []
 
 
