@@ -472,8 +472,14 @@ cudaError_t launch_adjoint(const void* G, const uint8_t* V, void* dV, int n, int
   e = ensure_smem_limit(reinterpret_cast<const void*>(adjoint_tc_kernel), kASmem);
   if (e != cudaSuccess) return e;
   const int grid = a.num_tiles < sm_count ? a.num_tiles : sm_count;
-  return launch_after(a.num_tiles <= 4 * sm_count, adjoint_tc_kernel, dim3(unsigned(grid)), dim3(kAThreads), kASmem, s, tmV, tmS,
-                      tmT, a);
+  // An early start saves about 2 us, which is lost in the runs' spread from four
+  // tiles per SM on.  Whole calls without / with it: 512 x 512 x 8 (0.9 tiles per
+  // SM) 30.7 / 26.7 us, 512 x 512 x 16 (1.7) 47.6 / 45.1, 1024 x 512 x 16 (3.5)
+  // 160.1 / 161.4, 2048 x 64 x 32 (3.5) 541.0 / 538.4, 2048 x 512 x 10 (4.3) 380.0 /
+  // 388.6, 2048 x 512 x 32 (13.8) 1145.2 / 1144.1.
+  const bool early = a.num_tiles <= 4 * sm_count;
+  return launch_after(early, adjoint_tc_kernel, dim3(unsigned(grid)), dim3(kAThreads), kASmem, s,
+                      tmV, tmS, tmT, a);
 }
 
 }  // namespace ftdx

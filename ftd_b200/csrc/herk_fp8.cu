@@ -897,9 +897,12 @@ __global__ void __launch_bounds__(kFused ? kFusedThreads : kHerkThreads, 1)
 //   MMA 1: A = Re_j, B = [Re_i | Im_i]   -> Re += Re_j Re_i, Im += Re_j Im_i
 //   MMA 2: A = Im_j, B = [Im_i | -Re_i]  -> Re += Im_j Im_i, Im -= Im_j Re_i
 // so the leader loads (Re_i, Im_i) and the partner (Im_i, -Re_i), the third
-// operand plane holding -Re.  Two MMAs per 32 samples instead of four of
-// N = 128: each MMA reads half as many operand bytes per multiply-add from
-// shared memory, which bounds the single-CTA kernel.  The leader CTA (rank 0)
+// operand plane holding -Re.  Two MMAs per 32 samples instead of the
+// single-CTA kernel's three: a CTA's shared memory gives 512 operand rows instead
+// of 896 for the same multiply-adds, and takes the same 64 KB of loads per
+// k-block.  That is not what sets this kernel's pace, though: 1880 clocks per
+// k-block and CTA against 1630 (tensor pipe 54% and 63% busy, 4096 inputs x 8
+// channels x 1024); what does is not found.  The leader CTA (rank 0)
 // owns the full barriers (the partner's loads count their bytes there) and
 // issues the MMAs; each commit arrives on the matching barrier of both CTAs
 // (one multicast commit);

@@ -192,7 +192,8 @@ void set_thread_error(const char* fmt, ...);
 // to FP16 take 30.6 us without and 26.7 with an early start, 16 of 1024 x 1024
 // FP16 samples 59.4 and 58.1.  Kernels of 200 us and more lose 0.5 to 1% by it
 // (their blocks take their SMs in the order in which the kernel before leaves
-// them), so callers ask for it up to kEarlyKBlocks k-blocks per SM.
+// them), so the correlators ask for it up to kEarlyKBlocks k-blocks per SM; the
+// float quantiser and the adjoint have lines of their own (precision.cu, adjoint.cu).
 constexpr int64_t kEarlyKBlocks = 64;
 template <typename... KArgs, typename... Args>
 cudaError_t launch_after(bool early, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,

@@ -463,11 +463,14 @@ cudaError_t launch_float_to_planes(const void* a, uint8_t* z, int64_t rows, int 
   // The cooperative kernel takes a step per channel, each with a wait for the
   // whole grid, and saves the second read from HBM: it needs a channel that is
   // long against the wait, or a single one.  Promotion in us, cooperative / two
-  // kernels: 16 channels of 33.6 MB 178 / 220, 4 of them 56 / 67, one of them
-  // 18.2 / 18.7, one of 5.6 MB 11.7 / 12.1; before either loaded whole spans: 8
-  // channels of 16.8 MB 76 / 71, 16 of 8.4 MB 70 / 64, of 4.2 MB 54 / 30, of 1.2
-  // MB 47 / 19.  The split mode (hi and lo columns) was
-  // slower on it at any size: 1.02 against 0.91 ms at 4096 x 64 x 1024.
+  // kernels: one channel of 1.2 MB 10.3 / 10.9, of 8.4 MB 12.4 / 12.7, of 33.6 MB
+  // 18.5 / 21.0; 16 of 1.2 MB 49 / 16, of 4.2 MB 56 / 35; 4 of 8.4 MB 22 / 19, 16 of
+  // them 67 / 66; 8 of 16.8 MB 57 / 68, of 22.9 MB 70 / 88; 16 of 33.6 MB 181 / 223.
+  // So the two meet between 9 and 12 MB; the line at 24 MB is where they met before
+  // either loaded whole spans (8 of 16.8 MB 76 / 71 then), and calls of 12 to 24
+  // MB a channel run up to 16% above what the other choice gives.  The split mode
+  // (hi and lo columns) was slower on it at any size: 1.02 against 0.91 ms at
+  // 4096 x 64 x 1024.
   const bool large = batch == 1 || int64_t(n) * K * int64_t(sizeof(float2)) >= 24000000;
   const int per_sm = split || !large ? 0 : scale_quantize_blocks_per_sm();
   if (per_sm > 0 && adjacent && (reinterpret_cast<uintptr_t>(arrive) & 127) == 0 &&
@@ -497,8 +500,12 @@ cudaError_t launch_float_to_planes(const void* a, uint8_t* z, int64_t rows, int 
   if (e != cudaSuccess) return e;
   const int rpb = promotion_rows_per_block(rows, Kp >> 3);
   const int64_t blocks = (rows + rpb - 1) / rpb;
-  e = launch_after(rows * K <= (int64_t(8) << 20), quantize_kernel, dim3(unsigned(blocks)), dim3(256), 0, s,
-                   static_cast<const float2*>(a), z, rows, K, Kp, zpitch, n, amax_bits, out_scale,
+  // An early start saves about 2 us: whole calls without / with it, 2 channels of
+  // 1024 x 1024 26.6 / 24.4 us, 8 of them (the line, 8 M samples) 51.3 / 49.4, 16
+  // 100.3 / 98.0, hi + lo 160.9 / 158.2; past the line the gain is below what runs
+  // differ by (hi + lo, 16 channels of 4096 x 1024: 1451 / 1549, 32: 3023 / 3019).
+  const bool early = rows * K <= (int64_t(8) << 20);
+  e = launch_after(early, quantize_kernel, dim3(unsigned(blocks)), dim3(256), 0, s, static_cast<const float2*>(a), z, rows, K, Kp, zpitch, n, amax_bits, out_scale,
                    split, rpb, vec);
   if (e == cudaSuccess && neg) e = launch_negate_plane(z, rows * zpitch, sm_count, s);
   return e;

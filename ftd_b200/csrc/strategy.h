@@ -71,6 +71,14 @@ inline size_t split_bytes(int N, int batch, int splits) {
 // apart, 8.0 fused in; 1024 x 1024 x 16 (576 tiles): 41.1 apart, 43.5 fused in.
 // The choice depends on sizes and on `fused` alone, so that a call prepared
 // for capture (ftdx_init_herk) finds its plan.
+// It also decides for FP16 and FP32 input and for hi + lo, whose promotion costs
+// more and whose k-blocks take three products: it then splits too little, never
+// where unsplit is faster.  Rule / best split / unsplit, us, promotion apart:
+// FP16 128 x 2048 x 4 14.5 / 12.5 / 18.6, 256 x 16384 x 4 37.4 / 37.2 / 95.3; FP8 of
+// floats 512 x 8192 x 1 28.9 / 28.9 / 55.6; hi + lo 300 x 1024 x 1 30.9 / 20.6 / 30.9,
+// 256 x 4096 x 2 29.8 / 27.0 / 78.0, 512 x 8192 x 1 44.5 / 41.1 / 142.3.  Of 36 such
+// shapes 28 are within 8% of the best; the others have at most six tiles, and the
+// worst (hi + lo, one tile of 8 k-blocks) takes 28.8 us where 17.2 could be had.
 inline Strategy auto_strategy(int sm_count, int N, int K, int batch, bool fused_ok,
                               bool split_ok) {
   const int64_t nb = (N + kTile - 1) / kTile, tiles = nb * (nb + 1) / 2 * batch;
