@@ -377,7 +377,7 @@ FTDX_API int ftdx_graph_count(ftdx_handle h);
 FTDX_API ftdx_status ftdx_set_strategy(ftdx_handle h, int store_mode, int grid);
 
 /* Back to a new handle's state: the call's sizes decide again (strategy and
- * split count). */
+ * split count).  No counterpart in the reference, nor has the next one. */
 FTDX_API ftdx_status ftdx_clear_strategy(ftdx_handle h);
 
 /* The strategy that the last correlator call on this handle launched, however
